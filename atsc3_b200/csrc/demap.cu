@@ -14,12 +14,9 @@
 // The |z|^2 term common to every point cancels in a_i - b_i
 // (lab/m16_demap_fast.py:27-58), so it is only used by the sigma2 estimator.
 //
-// Work split: one thread per cell; the alphabet (Re, Im, |p|^2, 3*M floats)
-// is staged in shared memory; cells (float2) and per-cell sigma2 are read
-// coalesced.  Per-bit minima: labels are walked in blocks of 16; the four
-// low label bits are compile-time constants inside a block, the high bits
-// are constant across it and take the block minimum once.  This is the
-// point-distance work of K=2 -- no tensor-core shape.
+// Work split: one thread per cell; the alphabet (Re, Im,
+// |p|^2, 3*M values) is staged in shared memory; cells and per-cell sigma2 are
+// read coalesced.  The point distance is work of K=2: no tensor-core shape.
 
 #include <cuda_runtime.h>
 
@@ -29,37 +26,102 @@
 
 namespace atsc3 {
 
-template <int NB>
-__global__ void __launch_bounds__(256) demap_kernel(
-    const float2 *__restrict__ cells, int64_t ld_cells, int nblk, int ncell,
-    const float *__restrict__ pts, int sigma_mode,
-    const float *__restrict__ sigma2, int64_t ld_sigma, float s2scalar,
-    const int32_t *__restrict__ lam_of_q, float *__restrict__ out,
+constexpr int DEMAP_T = 256;    // threads per CTA, a cell each
+// CTAs per SM the compiler has to leave room for: the fully unrolled 64- and
+// 256-point kernels run best with just the registers of four (75 x 64800-bit
+// Blocks: 64 points 31.2 us without the bound, 23.0 with it; 256 points 37.4
+// and 31.6; 16 points and the grids lose by it)
+template <int NB, typename T>
+constexpr int demap_ctas() { return sizeof(T) == 4 && (NB == 6 || NB == 8) ? 4 : 1; }
+
+// Writes one cell's LLRs: through lam_of_q (nullable) or in transmission
+// order, the table and the contiguous LLRs in the widest aligned pieces.
+template <int NB, typename T>
+__device__ __forceinline__ void store_llrs(const T (&d)[NB], int s,
+                                           const int32_t *__restrict__ lam_of_q,
+                                           T *__restrict__ o) {
+  const int q0 = s * NB;
+  if (lam_of_q) {
+    int32_t at[NB];
+    if (NB % 4 == 0 && (reinterpret_cast<uintptr_t>(lam_of_q) & 15) == 0) {
+#pragma unroll
+      for (int i = 0; i + 4 <= NB; i += 4) {
+        const int4 v = __ldg(reinterpret_cast<const int4 *>(lam_of_q + q0 + i));
+        at[i] = v.x;
+        at[i + 1] = v.y;
+        at[i + 2] = v.z;
+        at[i + 3] = v.w;
+      }
+    } else if ((reinterpret_cast<uintptr_t>(lam_of_q) & 7) == 0) {
+#pragma unroll
+      for (int i = 0; i < NB; i += 2) {
+        const int2 v = __ldg(reinterpret_cast<const int2 *>(lam_of_q + q0 + i));
+        at[i] = v.x;
+        at[i + 1] = v.y;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < NB; ++i) at[i] = __ldg(lam_of_q + q0 + i);
+    }
+#pragma unroll
+    for (int i = 0; i < NB; ++i) o[at[i]] = d[i];
+    return;
+  }
+  T *r = o + q0;
+  if (sizeof(T) == 4 && (reinterpret_cast<uintptr_t>(r) & 7) == 0) {
+#pragma unroll
+    for (int i = 0; i < NB; i += 2)
+      *reinterpret_cast<float2 *>(r + i) = make_float2((float)d[i], (float)d[i + 1]);
+  } else if (sizeof(T) == 8 && (reinterpret_cast<uintptr_t>(r) & 15) == 0) {
+#pragma unroll
+    for (int i = 0; i < NB; i += 2)
+      *reinterpret_cast<double2 *>(r + i) = make_double2(d[i], d[i + 1]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < NB; ++i) r[i] = d[i];
+  }
+}
+
+template <typename T> struct Cell2;
+template <> struct Cell2<float> { using type = float2; };
+template <> struct Cell2<double> { using type = double2; };
+
+// T = float: the decode path; T = double: the drop-in for the reference's
+// default float64 demap_llr_fast (lab/m16_demap_fast.py:80-119).
+template <int NB, typename T>
+__global__ void __launch_bounds__(DEMAP_T, (demap_ctas<NB, T>())) demap_kernel(
+    const typename Cell2<T>::type *__restrict__ cells, int64_t ld_cells, int nblk,
+    int ncell, const T *__restrict__ pts, int sigma_mode,
+    const T *__restrict__ sigma2, int64_t ld_sigma, T s2scalar,
+    const int32_t *__restrict__ lam_of_q, T *__restrict__ out,
     int64_t ld_out) {
-  constexpr int M = 1 << NB;
-  extern __shared__ float sp[];
-  float *spr = sp, *spi = sp + M, *sp2 = sp + 2 * M;
-  for (int k = threadIdx.x; k < 3 * M; k += blockDim.x) sp[k] = pts[k];
-  __syncthreads();
+  using A = DemapArith<T>;
+  extern __shared__ __align__(16) unsigned char demap_smem[];
+  T *sp = reinterpret_cast<T *>(demap_smem);
+  const int form = stage_points<NB, T>(sp, pts);
   const int64_t total = (int64_t)nblk * ncell;
-  for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < total;
-       g += (int64_t)gridDim.x * blockDim.x) {
-    const int b = (int)(g / ncell);
-    const int s = (int)(g - (int64_t)b * ncell);
-    const float2 z = cells[(size_t)b * ld_cells + s];
-    float mn[NB][2];
-    cell_minima<NB>(z.x, z.y, spr, spi, sp2, mn, nullptr);
-    float s2 = s2scalar;
+  for (int64_t g0 = (int64_t)blockIdx.x * DEMAP_T; g0 < total;
+       g0 += (int64_t)gridDim.x * DEMAP_T) {
+    // the CTA's first cell, then a 32-bit step from it
+    const int64_t b0 = g0 / ncell;
+    const uint32_t x = (uint32_t)(g0 - b0 * ncell) + threadIdx.x;
+    const uint32_t step = x / (uint32_t)ncell;
+    const int64_t b = b0 + step;
+    const int s = (int)(x - step * (uint32_t)ncell);
+    if (b >= nblk) break;
+    const typename Cell2<T>::type z = cells[(size_t)b * ld_cells + s];
+    T mn[NB][2];
+    cell_minima<NB, T>(z.x, z.y, sp, form, mn);
+    T s2 = s2scalar;
     if (sigma_mode == 1) s2 = sigma2[(size_t)b * ld_sigma + s];
     else if (sigma_mode == 2) s2 = sigma2[b];
-    float *o = out + (size_t)b * ld_out;
+    T d[NB];
 #pragma unroll
     for (int i = 0; i < NB; ++i) {
-      float d = __fsub_rn(mn[i][1], mn[i][0]);
-      if (sigma_mode != 3) d = __fdiv_rn(d, s2);
-      const int q = s * NB + i;
-      o[lam_of_q ? __ldg(lam_of_q + q) : q] = d;
+      d[i] = A::sub(mn[i][1], mn[i][0]);
+      if (sigma_mode != 3) d[i] = A::div(d[i], s2);
     }
+    store_llrs<NB, T>(d, s, lam_of_q, out + (size_t)b * ld_out);
   }
 }
 
@@ -68,18 +130,17 @@ template <int NB>
 __global__ void __launch_bounds__(256) row_sigma_kernel(
     const float2 *__restrict__ cells, int64_t ld_cells, int ncell,
     const float *__restrict__ pts, float *__restrict__ sigma2) {
-  constexpr int M = 1 << NB;
-  extern __shared__ float sp[];
+  extern __shared__ __align__(16) unsigned char demap_smem[];
   __shared__ double red[32];
-  float *spr = sp, *spi = sp + M, *sp2 = sp + 2 * M;
-  for (int k = threadIdx.x; k < 3 * M; k += blockDim.x) sp[k] = pts[k];
-  __syncthreads();
+  float *sp = reinterpret_cast<float *>(demap_smem);
+  const int form = stage_points<NB, float>(sp, pts);
   const int b = blockIdx.x;
   double acc = 0.0;
   for (int s = threadIdx.x; s < ncell; s += blockDim.x) {
     const float2 z = cells[(size_t)b * ld_cells + s];
-    float mn[NB][2], qmin;
-    cell_minima<NB>(z.x, z.y, spr, spi, sp2, mn, &qmin);
+    float mn[NB][2];
+    cell_minima<NB, float>(z.x, z.y, sp, form, mn);
+    const float qmin = fminf(mn[0][0], mn[0][1]);
     const float z2 = __fadd_rn(__fmul_rn(z.x, z.x), __fmul_rn(z.y, z.y));
     acc += (double)__fadd_rn(z2, qmin);
   }
@@ -94,44 +155,6 @@ __global__ void __launch_bounds__(256) row_sigma_kernel(
   }
 }
 
-// ---- float64: the drop-in for the reference's default float64
-// demap_llr_fast (lab/m16_demap_fast.py:80-119; m = |p|^2 - 2 Re(y p*), the
-// per-bit minima, / sigma2).  Same work split, double arithmetic, cells as
-// double2 (complex128), output in q order or through lam_of_q.
-template <int NB>
-__global__ void __launch_bounds__(256) demap_f64_kernel(
-    const double2 *__restrict__ cells, int64_t ld_cells, int nblk, int ncell,
-    const double *__restrict__ pts, int sigma_mode,
-    const double *__restrict__ sigma2, int64_t ld_sigma, double s2scalar,
-    const int32_t *__restrict__ lam_of_q, double *__restrict__ out,
-    int64_t ld_out) {
-  using A = DemapArith<double>;
-  constexpr int M = 1 << NB;
-  extern __shared__ double spd[];
-  double *spr = spd, *spi = spd + M, *sp2 = spd + 2 * M;
-  for (int k = threadIdx.x; k < 3 * M; k += blockDim.x) spd[k] = pts[k];
-  __syncthreads();
-  const int64_t total = (int64_t)nblk * ncell;
-  for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < total;
-       g += (int64_t)gridDim.x * blockDim.x) {
-    const int b = (int)(g / ncell);
-    const int s = (int)(g - (int64_t)b * ncell);
-    const double2 z = cells[(size_t)b * ld_cells + s];
-    double mn[NB][2];
-    cell_minima<NB, double>(z.x, z.y, spr, spi, sp2, mn, nullptr);
-    double s2 = s2scalar;
-    if (sigma_mode == 1) s2 = sigma2[(size_t)b * ld_sigma + s];
-    else if (sigma_mode == 2) s2 = sigma2[b];
-    double *o = out + (size_t)b * ld_out;
-#pragma unroll
-    for (int i = 0; i < NB; ++i) {
-      const double d = A::div(A::sub(mn[i][1], mn[i][0]), s2);
-      const int q = s * NB + i;
-      o[lam_of_q ? __ldg(lam_of_q + q) : q] = d;
-    }
-  }
-}
-
 // sigma2[b] = max(mean_s(|z|^2 + min_k q_k), 1e-9) in float64 (the estimate
 // of lab/m16_demap_fast.py:104-106).
 template <int NB>
@@ -139,18 +162,17 @@ __global__ void __launch_bounds__(256) row_sigma_f64_kernel(
     const double2 *__restrict__ cells, int64_t ld_cells, int ncell,
     const double *__restrict__ pts, double *__restrict__ sigma2) {
   using A = DemapArith<double>;
-  constexpr int M = 1 << NB;
-  extern __shared__ double spd[];
+  extern __shared__ __align__(16) unsigned char demap_smem[];
   __shared__ double red[32];
-  double *spr = spd, *spi = spd + M, *sp2 = spd + 2 * M;
-  for (int k = threadIdx.x; k < 3 * M; k += blockDim.x) spd[k] = pts[k];
-  __syncthreads();
+  double *sp = reinterpret_cast<double *>(demap_smem);
+  const int form = stage_points<NB, double>(sp, pts);
   const int b = blockIdx.x;
   double acc = 0.0;
   for (int s = threadIdx.x; s < ncell; s += blockDim.x) {
     const double2 z = cells[(size_t)b * ld_cells + s];
-    double mn[NB][2], qmin;
-    cell_minima<NB, double>(z.x, z.y, spr, spi, sp2, mn, &qmin);
+    double mn[NB][2];
+    cell_minima<NB, double>(z.x, z.y, sp, form, mn);
+    const double qmin = A::min(mn[0][0], mn[0][1]);
     const double z2 = A::add(A::mul(z.x, z.x), A::mul(z.y, z.y));
     acc += A::add(z2, qmin);
   }
@@ -172,12 +194,12 @@ typedef void (*SigmaF64Fn)(const double2 *, int64_t, int, const double *,
 
 static DemapF64Fn demap_f64_fn(int nb) {
   switch (nb) {
-    case 2: return demap_f64_kernel<2>;
-    case 4: return demap_f64_kernel<4>;
-    case 6: return demap_f64_kernel<6>;
-    case 8: return demap_f64_kernel<8>;
-    case 10: return demap_f64_kernel<10>;
-    case 12: return demap_f64_kernel<12>;
+    case 2: return demap_kernel<2, double>;
+    case 4: return demap_kernel<4, double>;
+    case 6: return demap_kernel<6, double>;
+    case 8: return demap_kernel<8, double>;
+    case 10: return demap_kernel<10, double>;
+    case 12: return demap_kernel<12, double>;
   }
   return nullptr;
 }
@@ -201,12 +223,12 @@ typedef void (*SigmaFn)(const float2 *, int64_t, int, const float *, float *);
 
 static DemapFn demap_fn(int nb) {
   switch (nb) {
-    case 2: return demap_kernel<2>;
-    case 4: return demap_kernel<4>;
-    case 6: return demap_kernel<6>;
-    case 8: return demap_kernel<8>;
-    case 10: return demap_kernel<10>;
-    case 12: return demap_kernel<12>;
+    case 2: return demap_kernel<2, float>;
+    case 4: return demap_kernel<4, float>;
+    case 6: return demap_kernel<6, float>;
+    case 8: return demap_kernel<8, float>;
+    case 10: return demap_kernel<10, float>;
+    case 12: return demap_kernel<12, float>;
   }
   return nullptr;
 }
@@ -222,6 +244,11 @@ static SigmaFn sigma_fn(int nb) {
   }
   return nullptr;
 }
+
+// CTAs per SM at most: enough for the hardware to even out the last wave; where
+// staging the alphabet costs as much as demapping a CTA's cells (12 or 48 KB of
+// grid points, a few labels formed per cell), no more than are resident at once.
+static int demap_waves(int nbits) { return nbits >= 10 ? 3 : 32; }
 
 static int num_sms() {
   static int sms = 0;
@@ -251,19 +278,19 @@ int32_t demap_launch(const float *cells, int64_t ld_cells, int nblk, int ncell,
   ATSC3_ARG(!(sigma_mode == 1 || sigma_mode == 2) || sigma2 != nullptr,
             "sigma2 array required");
   ATSC3_ARG(sigma_mode != 1 || ld_sigma >= ncell, "ld_sigma < ncell");
-  const int smem = 3 * (1 << nbits) * 4;
+  const int smem = demap_smem_bytes(nbits, 4);
   if (smem > 48 * 1024)
     ATSC3_CUDA(cudaFuncSetAttribute((const void *)fn,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     smem));
   const int64_t total = (int64_t)nblk * ncell;
-  int64_t grid = (total + 255) / 256;
-  const int64_t cap = (int64_t)num_sms() * 8;
+  int64_t grid = (total + DEMAP_T - 1) / DEMAP_T;
+  const int64_t cap = (int64_t)num_sms() * demap_waves(nbits);
   if (grid > cap) grid = cap;
-  fn<<<(unsigned)grid, 256, smem, st>>>((const float2 *)cells, ld_cells, nblk,
-                                        ncell, pts, sigma_mode, sigma2,
-                                        ld_sigma, s2scalar, lam_of_q, out,
-                                        ld_out);
+  fn<<<(unsigned)grid, DEMAP_T, smem, st>>>((const float2 *)cells, ld_cells, nblk,
+                                       ncell, pts, sigma_mode, sigma2,
+                                       ld_sigma, s2scalar, lam_of_q, out,
+                                       ld_out);
   ATSC3_CUDA(cudaGetLastError());
   return 0;
 }
@@ -285,19 +312,19 @@ int32_t demap_f64_launch(const double *cells, int64_t ld_cells, int nblk,
   ATSC3_ARG(((uintptr_t)cells & 15) == 0, "cells must be 16-byte aligned");
   ATSC3_ARG(sigma_mode == 0 || sigma2 != nullptr, "sigma2 array required");
   ATSC3_ARG(sigma_mode != 1 || ld_sigma >= ncell, "ld_sigma < ncell");
-  const int smem = 3 * (1 << nbits) * 8;
+  const int smem = demap_smem_bytes(nbits, 8);
   if (smem > 48 * 1024)
     ATSC3_CUDA(cudaFuncSetAttribute((const void *)fn,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     smem));
   const int64_t total = (int64_t)nblk * ncell;
-  int64_t grid = (total + 255) / 256;
-  const int64_t cap = (int64_t)num_sms() * 8;
+  int64_t grid = (total + DEMAP_T - 1) / DEMAP_T;
+  const int64_t cap = (int64_t)num_sms() * demap_waves(nbits);
   if (grid > cap) grid = cap;
-  fn<<<(unsigned)grid, 256, smem, st>>>((const double2 *)cells, ld_cells, nblk,
-                                        ncell, pts, sigma_mode, sigma2,
-                                        ld_sigma, s2scalar, lam_of_q, out,
-                                        ld_out);
+  fn<<<(unsigned)grid, DEMAP_T, smem, st>>>((const double2 *)cells, ld_cells, nblk,
+                                       ncell, pts, sigma_mode, sigma2,
+                                       ld_sigma, s2scalar, lam_of_q, out,
+                                       ld_out);
   ATSC3_CUDA(cudaGetLastError());
   return 0;
 }
@@ -312,7 +339,7 @@ int32_t row_sigma_f64_launch(const double *cells, int64_t ld_cells, int nblk,
   ATSC3_ARG(cells && pts && sigma2, "null pointer");
   ATSC3_ARG(ld_cells >= ncell, "ld_cells < ncell");
   ATSC3_ARG(((uintptr_t)cells & 15) == 0, "cells must be 16-byte aligned");
-  const int smem = 3 * (1 << nbits) * 8;
+  const int smem = demap_smem_bytes(nbits, 8);
   if (smem > 48 * 1024)
     ATSC3_CUDA(cudaFuncSetAttribute((const void *)fn,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -332,7 +359,7 @@ int32_t row_sigma_launch(const float *cells, int64_t ld_cells, int nblk,
   if (nblk == 0) return 0;
   ATSC3_ARG(cells && pts && sigma2, "null pointer");
   ATSC3_ARG(((uintptr_t)cells & 7) == 0, "cells must be 8-byte aligned");
-  const int smem = 3 * (1 << nbits) * 4;
+  const int smem = demap_smem_bytes(nbits, 4);
   if (smem > 48 * 1024)
     ATSC3_CUDA(cudaFuncSetAttribute((const void *)fn,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -365,30 +392,25 @@ struct DemapBatchArgs {
 
 template <int NB>
 __device__ __forceinline__ void demap_cell_batch(const DemapBatchArgs &a, int b,
-                                                 int s, const float *sp) {
-  constexpr int M = 1 << NB;
+                                                 int s, float *sp) {
+  const int form = stage_points<NB, float>(sp, a.pts + a.pts_off[b]);
+  if (s >= a.ncell[b]) return;
   const float2 z = a.cells[a.cell_off[b] + s];
   float mn[NB][2];
-  cell_minima<NB>(z.x, z.y, sp, sp + M, sp + 2 * M, mn, nullptr);
+  cell_minima<NB, float>(z.x, z.y, sp, form, mn);
   const float s2 = a.sigma2[b];
-  const int32_t *lq = a.lq + a.lq_off[b];
-  float *o = a.llr + a.llr_off[b];
+  float d[NB];
 #pragma unroll
-  for (int i = 0; i < NB; ++i)
-    o[__ldg(lq + s * NB + i)] = __fdiv_rn(__fsub_rn(mn[i][1], mn[i][0]), s2);
+  for (int i = 0; i < NB; ++i) d[i] = __fdiv_rn(__fsub_rn(mn[i][1], mn[i][0]), s2);
+  store_llrs<NB, float>(d, s, a.lq + a.lq_off[b], a.llr + a.llr_off[b]);
 }
 
 __global__ void __launch_bounds__(256) demap_batch_kernel(const DemapBatchArgs a) {
-  extern __shared__ float sp[];
+  extern __shared__ __align__(16) unsigned char demap_smem[];
+  float *sp = reinterpret_cast<float *>(demap_smem);
   const int b = a.chunk_blk[blockIdx.x];
   const int s = a.chunk_start[blockIdx.x] + threadIdx.x;
-  const int nb = a.nbits[b];
-  const int M3 = 3 << nb;
-  const float *src = a.pts + a.pts_off[b];
-  for (int k = threadIdx.x; k < M3; k += blockDim.x) sp[k] = src[k];
-  __syncthreads();
-  if (s >= a.ncell[b]) return;
-  switch (nb) {
+  switch (a.nbits[b]) {
     case 2: demap_cell_batch<2>(a, b, s, sp); break;
     case 4: demap_cell_batch<4>(a, b, s, sp); break;
     case 6: demap_cell_batch<6>(a, b, s, sp); break;
@@ -417,7 +439,7 @@ int32_t atsc3_demap_batch(const float *cells, const int64_t *cell_off,
                 lq && lq_off && llr && llr_off && chunk_blk && chunk_start,
             "null pointer");
   ATSC3_ARG(max_nbits >= 2 && max_nbits <= 12, "max_nbits must be 2..12");
-  const int smem = 3 * (1 << max_nbits) * 4;
+  const int smem = demap_smem_bytes(max_nbits, 4);
   if (smem > 48 * 1024)
     ATSC3_CUDA(cudaFuncSetAttribute((const void *)demap_batch_kernel,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, smem));

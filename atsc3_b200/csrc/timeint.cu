@@ -64,11 +64,9 @@ __device__ __forceinline__ int64_t gather_source(const GatherArgs &a, int b,
 
 template <int NB>
 __global__ void __launch_bounds__(256) demap_gather_kernel(const GatherArgs a) {
-  constexpr int M = 1 << NB;
-  extern __shared__ float sp[];
-  float *spr = sp, *spi = sp + M, *sp2 = sp + 2 * M;
-  for (int k = threadIdx.x; k < 3 * M; k += blockDim.x) sp[k] = a.pts[k];
-  __syncthreads();
+  extern __shared__ __align__(16) unsigned char demap_smem[];
+  float *sp = reinterpret_cast<float *>(demap_smem);
+  const int form = stage_points<NB, float>(sp, a.pts);
   const int64_t total = (int64_t)a.nblk * a.ncell;
   for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < total;
        g += (int64_t)gridDim.x * blockDim.x) {
@@ -86,7 +84,7 @@ __global__ void __launch_bounds__(256) demap_gather_kernel(const GatherArgs a) {
     }
     const float2 z = a.cells[src];
     float mn[NB][2];
-    cell_minima<NB>(z.x, z.y, spr, spi, sp2, mn, nullptr);
+    cell_minima<NB, float>(z.x, z.y, sp, form, mn);
     float s2 = a.s2scalar;
     if (a.sigma_mode == 1) s2 = a.sigma2[src];
     else if (a.sigma_mode == 2) s2 = a.sigma2[b];
@@ -159,7 +157,7 @@ int32_t atsc3_demap_gather(const float *cells, int64_t ncells, int32_t nblk,
   a.lam_of_q = lam_of_q;
   a.out = out;
   a.ld_out = ld_out;
-  const int smem = 3 * (1 << nbits) * 4;
+  const int smem = demap_smem_bytes(nbits, 4);
   if (smem > 48 * 1024)
     ATSC3_CUDA(cudaFuncSetAttribute((const void *)fn,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -99,11 +99,14 @@ def demap(cells, mod, rate, sigma2=None, n=None, deinterleave=True, out=None,
     s2s = 0.0
     ld_s = 0
     if sigma2 is None:
-        s2t = torch.empty(nblk, dtype=torch.float32, device=dev)
-        N.call("atsc3_demap_row_sigma2", zf.data_ptr(), zf.stride(0) // 2,
-               nblk, ncell, pts.data_ptr(), nb, s2t.data_ptr(), st)
-        mode = 2
-    elif isinstance(sigma2, (float, int, np.floating)):
+        work = torch.empty(max(nblk, 4096), dtype=torch.float64, device=dev)
+        N.call("atsc3_demap_estimate", zf.data_ptr(), zf.stride(0) // 2, nblk,
+               ncell, pts.data_ptr(), nb, N.ptr(lq), out.data_ptr(),
+               out.stride(0), work.data_ptr(), st)
+        if stream is not None:      # not the stream the allocator knows
+            out._demap_work = work
+        return out
+    if isinstance(sigma2, (float, int, np.floating)):
         mode, s2s = 0, float(np.float32(sigma2))
     else:
         s2t = sigma2.to(device=dev, dtype=torch.float32)
@@ -156,11 +159,14 @@ def demap_f64(cells, mod, rate, sigma2=None, n=None, deinterleave=False,
     st = stream if stream is not None else torch.cuda.current_stream(dev).cuda_stream
     s2t, s2s, ld_s = None, 0.0, 0
     if sigma2 is None:
-        s2t = torch.empty(nblk, dtype=torch.float64, device=dev)
-        N.call("atsc3_demap_row_sigma2_f64", zf.data_ptr(), zf.stride(0) // 2,
-               nblk, ncell, pts.data_ptr(), nb, s2t.data_ptr(), st)
-        mode = 2
-    elif isinstance(sigma2, (float, int, np.floating)):
+        work = torch.empty(max(nblk, 4096), dtype=torch.float64, device=dev)
+        N.call("atsc3_demap_estimate_f64", zf.data_ptr(), zf.stride(0) // 2,
+               nblk, ncell, pts.data_ptr(), nb, N.ptr(lq), out.data_ptr(),
+               out.stride(0), work.data_ptr(), st)
+        if stream is not None:      # not the stream the allocator knows
+            out._demap_work = work
+        return out
+    if isinstance(sigma2, (float, int, np.floating)):
         mode, s2s = 0, float(sigma2)
     else:
         s2t = sigma2.to(device=dev, dtype=torch.float64).reshape(nblk, ncell)

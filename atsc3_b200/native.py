@@ -138,6 +138,10 @@ SIGNATURES = {
                                 c_vp, c_i64, c_f64, c_vp, c_vp, c_i64, c_vp]),
     "atsc3_demap_row_sigma2_f64": (c_i32, [c_vp, c_i64, c_i32, c_i32, c_vp,
                                            c_i32, c_vp, c_vp]),
+    "atsc3_demap_estimate": (c_i32, [c_vp, c_i64, c_i32, c_i32, c_vp, c_i32,
+                                     c_vp, c_vp, c_i64, c_vp, c_vp]),
+    "atsc3_demap_estimate_f64": (c_i32, [c_vp, c_i64, c_i32, c_i32, c_vp, c_i32,
+                                         c_vp, c_vp, c_i64, c_vp, c_vp]),
     "atsc3_bch_check": (c_i32, [c_vp, c_i64, c_i32, c_i32, c_vp, c_vp, c_vp,
                                 c_vp, c_i32, c_vp, c_i64, c_vp]),
     "atsc3_bch_syndrome_bits": (c_i32, [c_vp, c_i64, c_i32, c_i32, c_vp,

@@ -536,6 +536,20 @@ int32_t atsc3_demap_row_sigma2_f64(const double *cells, int64_t ld_cells,
                                    const double *pts, int32_t nbits,
                                    double *sigma2, void *stream);
 
+/* The demapper with sigma2 estimated per row (as atsc3_demap_row_sigma2 and
+ * its float64 form estimate it), the minima formed once for both: otherwise as
+ * atsc3_demap / atsc3_demap_f64 with sigma_mode 2.  lam_of_q (nullable) is a
+ * permutation of 0 .. ncell*nbits-1.  work: device, 8-byte aligned,
+ * 8 * max(nblk, 4096) bytes. */
+int32_t atsc3_demap_estimate(const float *cells, int64_t ld_cells, int32_t nblk,
+                             int32_t ncell, const float *pts, int32_t nbits,
+                             const int32_t *lam_of_q, float *out, int64_t ld_out,
+                             void *work, void *stream);
+int32_t atsc3_demap_estimate_f64(const double *cells, int64_t ld_cells, int32_t nblk,
+                                 int32_t ncell, const double *pts, int32_t nbits,
+                                 const int32_t *lam_of_q, double *out, int64_t ld_out,
+                                 void *work, void *stream);
+
 /* BCH zero-syndrome check (A/322 6.1.2.1) plus descramble of the payload.
  * hard: (nblk, ld_hard) packed hard decisions (as atsc3_ldpc_decode_flood
  *   writes them); the first kldpc bits are the BCH codeword.

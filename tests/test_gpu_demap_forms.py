@@ -53,3 +53,40 @@ def test_demap_forms_vs_oracle(mod, f64, moved):
         N.call(name, torch.view_as_real(zt).data_ptr(), n, 2, n, t.data_ptr(), nb, 0, None, 0, 1.0,
                None, out.data_ptr(), n * nb, torch.cuda.current_stream().cuda_stream)
         assert np.array_equal(out.cpu().numpy().reshape(want.shape), want)
+
+
+@pytest.mark.parametrize("f64", [False, True])
+@pytest.mark.parametrize("mod,nblk,ncell,pad", [
+    ("QPSK", 5, 1, 0), ("16QAM", 3, 255, 1), ("64QAM", 1, 257, 3), ("256QAM", 2, 5000, 0),
+    ("1024QAM", 5000, 3, 0), ("4096QAM", 4, 700, 5)])
+def test_demap_estimate_rows(mod, nblk, ncell, pad, f64):
+    """sigma2 estimated per row: the undivided LLRs over the row's mean of
+    |z|^2 + min q.  The terms are the kernel's own roundings, summed here in
+    another order: (ncell + 4) roundings of the sum and the division (float64),
+    or one of the float32 mean and one of the division."""
+    import torch
+    from atsc3_b200 import demap as DM
+    nb = C.MOD_BITS[mod]
+    pts = np.array(C.alphabet(mod, "9/15"), np.complex128)
+    rng = np.random.default_rng(nblk)
+    z = pts[rng.integers(0, len(pts), (nblk, ncell))]
+    z = z + 0.05 * (rng.standard_normal(z.shape) + 1j * rng.standard_normal(z.shape))
+    z = z.astype(np.complex128 if f64 else np.complex64)
+    tab = (np.concatenate([pts.real, pts.imag, np.abs(pts) ** 2]) if f64
+           else np.concatenate(C.point_tables_f32(pts)).astype(np.float32)).reshape(3, -1)
+    near = np.empty((nblk, ncell))
+    for b in range(nblk):
+        zr, zi = z[b].real[:, None], z[b].imag[:, None]
+        q = (zr * tab[0] + zi * tab[1]) * tab.dtype.type(-2) + tab[2]
+        near[b] = z[b].real * z[b].real + z[b].imag * z[b].imag + q.min(1)
+    s2 = np.maximum(near.mean(1), 1e-9)[:, None]
+    fn, dt = (DM.demap_f64, torch.float64) if f64 else (DM.demap, torch.float32)
+    zt = torch.from_numpy(z).cuda()
+    raw = fn(zt, mod, "9/15", sigma2=1.0, deinterleave=False).cpu().numpy().astype(np.float64)
+    buf = torch.zeros((nblk, ncell * nb + pad), dtype=dt, device="cuda")
+    fn(zt, mod, "9/15", deinterleave=False, out=buf)
+    got = buf.cpu().numpy()
+    assert np.all(got[:, ncell * nb:] == 0)
+    want = raw / s2
+    tol = (ncell + 4) * 2.0 ** -53 if f64 else 2 * 2.0 ** -24 + ncell * 2.0 ** -53
+    assert np.all(np.abs(got[:, :ncell * nb] - want) <= tol * np.abs(want))

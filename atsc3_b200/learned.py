@@ -90,16 +90,18 @@ class WmsCode:
                   for k in ("cptr", "cidx", "vptr", "vedge", "vchk", "vpos",
                             "cbucket")}
 
-    def ptrs(self):
-        t = self.t
-        return [t[k].data_ptr() for k in ("cptr", "cidx", "vptr", "vedge",
-                                          "vchk", "vpos", "cbucket")]
+    def ptrs(self, keys=("cptr", "cidx", "vptr", "vedge", "vchk", "vpos",
+                         "cbucket")):
+        return [self.t[k].data_ptr() for k in keys]
 
     def init_params(self, iters, alpha=0.75, beta=0.0):
         torch = _torch()
         a = torch.full((iters, self.nbucket), float(alpha), device=self.dev)
         b = torch.full((iters, self.nbucket), float(beta), device=self.dev)
         return a, b
+
+
+_CSR = ("cptr", "cidx", "vptr", "vedge", "cbucket")
 
 
 class WeightedMinSum:
@@ -119,13 +121,16 @@ class WeightedMinSum:
                 llr = llr.contiguous()
                 a = alpha.detach().contiguous().float()
                 b = beta.detach().contiguous().float()
-                rec = torch.empty((iters, nblk, code.nc, 16), dtype=torch.uint8,
+                rec = torch.empty((iters, code.nc, nblk, 16), dtype=torch.uint8,
                                   device=llr.device)
                 out = torch.empty_like(llr)
-                N.call("atsc3_wms_forward", *code.ptrs(), code.n, code.nc,
-                       code.ne, code.nbucket, nblk, iters, llr.data_ptr(),
-                       a.data_ptr(), b.data_ptr(), int(bool(bf16)),
-                       rec.data_ptr(), out.data_ptr(),
+                work = torch.empty(nblk * (2 * code.n + code.ne),
+                                   dtype=torch.float32, device=llr.device)
+                N.call("atsc3_wms_forward_work", *code.ptrs(_CSR), code.n,
+                       code.nc, code.ne, code.nbucket, nblk, iters,
+                       llr.data_ptr(), a.data_ptr(), b.data_ptr(),
+                       int(bool(bf16)), rec.data_ptr(), out.data_ptr(),
+                       work.data_ptr(),
                        torch.cuda.current_stream(llr.device).cuda_stream)
                 ctx.save_for_backward(llr, a, b, rec)
                 ctx.code = code
@@ -136,13 +141,13 @@ class WeightedMinSum:
                 llr, a, b, rec = ctx.saved_tensors
                 code = ctx.code
                 iters, nblk = a.shape[0], llr.shape[0]
-                gt = g.contiguous().float().clone()
+                gt = g.contiguous().float()
                 ga = torch.zeros_like(a)
                 gb = torch.zeros_like(b)
                 work = torch.empty(nblk * code.n + 2 * nblk * code.ne,
                                    dtype=torch.float32, device=llr.device)
-                N.call("atsc3_wms_backward", *code.ptrs(), code.n, code.nc,
-                       code.ne, code.nbucket, nblk, iters, llr.data_ptr(),
+                N.call("atsc3_wms_gradients", *code.ptrs(_CSR), code.n, code.nc,
+                       code.ne, code.nbucket, nblk, iters,
                        a.data_ptr(), b.data_ptr(), rec.data_ptr(),
                        gt.data_ptr(), ga.data_ptr(), gb.data_ptr(),
                        work.data_ptr(),

@@ -113,6 +113,9 @@ SIGNATURES = {
     "atsc3_wms_forward": (c_i32, [c_vp] * 7 + [c_i32] * 6 + [c_vp, c_vp, c_vp,
                                                              c_i32, c_vp, c_vp,
                                                              c_vp]),
+    "atsc3_wms_forward_work": (c_i32, [c_vp] * 5 + [c_i32] * 6 + [c_vp, c_vp, c_vp,
+                                                                  c_i32] + [c_vp] * 4),
+    "atsc3_wms_gradients": (c_i32, [c_vp] * 5 + [c_i32] * 6 + [c_vp] * 8),
     "atsc3_wms_backward": (c_i32, [c_vp] * 7 + [c_i32] * 6 + [c_vp] * 9),
     "atsc3_ldpc_qc_decode_weighted": (c_i32, [c_vp, c_vp, c_i64, c_i32, c_i32,
                                               c_f32, c_i32, c_vp, c_vp, c_i32,

@@ -439,14 +439,32 @@ int32_t atsc3_ldpc_layered_inject_timeout(int32_t layer);
 /* ---- differentiable weighted min-sum ---------------------------------------
  * Unrolled flooding min-sum with per-iteration, per-check-degree scale and
  * offset: m = sgn * relu(alpha[t][d] * mu - beta[t][d]) (csrc/wms.cu).  No
- * reference counterpart.  Tables: device CSR (cptr, cidx, vptr, vedge), the
- * check and position of each variable-major edge (vchk, vpos), the bucket
- * of each check (int8, at most 127 buckets: its degree class, or its block
- * row for the per-row parameterisation).  records: (iters, nblk, nc) 16-byte per-check
- * checkpoints written by the forward and read by the backward.  Forward
- * writes tot_out = the posterior after `iters` iterations (no early stop).
- * Backward: gtot in = dL/dtot_out (overwritten), galpha/gbeta accumulate
- * (caller zeroes), work = nblk*n + 2*nblk*ne floats. */
+ * reference counterpart.  Tables: device CSR (cptr, cidx, vptr, vedge; checks of
+ * at most 32 edges), the check and position of each variable-major edge (vchk,
+ * vpos; not read), the bucket of each check (int8, at most 127 buckets: its
+ * degree class, or its block row for the per-row parameterisation).  records:
+ * (iters, nc, nblk) 16-byte per-check checkpoints written by the forward and read
+ * by the backward.  Forward writes tot_out = the posterior after `iters`
+ * iterations (no early stop).  atsc3_wms_forward_work takes its workspace,
+ * nblk * (2n + ne) floats, from the caller; atsc3_wms_forward takes it from the
+ * stream's memory pool.
+ * Backward: gtot in = dL/dtot_out (overwritten with dL/dllr), galpha/gbeta
+ * accumulate (caller zeroes), work = nblk*n + 2*nblk*ne floats.
+ * atsc3_wms_gradients: the parameter gradients alone, gtot is only read. */
+int32_t atsc3_wms_forward_work(const int32_t *cptr, const int32_t *cidx,
+                               const int32_t *vptr, const int32_t *vedge,
+                               const int8_t *cbucket, int32_t n, int32_t nc,
+                               int32_t ne, int32_t nbucket, int32_t nblk,
+                               int32_t iters, const float *llr, const float *alpha,
+                               const float *beta, int32_t bf16, void *records,
+                               float *tot_out, float *work, void *stream);
+int32_t atsc3_wms_gradients(const int32_t *cptr, const int32_t *cidx,
+                            const int32_t *vptr, const int32_t *vedge,
+                            const int8_t *cbucket, int32_t n, int32_t nc,
+                            int32_t ne, int32_t nbucket, int32_t nblk,
+                            int32_t iters, const float *alpha, const float *beta,
+                            const void *records, const float *gtot, float *galpha,
+                            float *gbeta, float *work, void *stream);
 int32_t atsc3_wms_forward(const int32_t *cptr, const int32_t *cidx,
                           const int32_t *vptr, const int32_t *vedge,
                           const int32_t *vchk, const int32_t *vpos,

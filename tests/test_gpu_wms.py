@@ -323,3 +323,29 @@ def test_row_weighted_training_step_gradients():
         gr = gr.numpy()
         rel = np.abs(g - gr).max() / max(np.abs(gr).max(), 1e-12)
         assert rel < 1e-2, rel
+
+
+@pytest.mark.parametrize("mode", ["degree", "row"])
+@pytest.mark.parametrize("nblk", [1, 3, 33])
+def test_wms_any_batch_vs_float64_reference(nblk, mode):
+    """Batches that are not whole warps, both bucket modes: the blocks-fastest
+    kernels against the float64 reference (the bars of the 4-block test)."""
+    import torch
+    from atsc3_b200.learned import WeightedMinSum, WmsCode, bce_loss, reference_f64
+    rate, n, T = "8/15", 16200, 3
+    lam, cw = _case(seed=nblk, nb=nblk, n=n)
+    code = WmsCode(rate, n, mode=mode)
+    rng = np.random.default_rng(nblk)
+    p0 = [(0.7 + 0.2 * rng.random((T, code.nbucket))).astype(np.float32),
+          (0.1 * rng.random((T, code.nbucket))).astype(np.float32)]
+    p = [torch.tensor(v, device="cuda", requires_grad=True) for v in p0]
+    p64 = [torch.tensor(v, dtype=torch.float64, requires_grad=True) for v in p0]
+    out = WeightedMinSum.apply(torch.from_numpy(lam).cuda(), *p, code, False)
+    bce_loss(out, torch.from_numpy(cw).cuda()).backward()
+    ref = reference_f64(torch.from_numpy(lam), *p64, rate, n, mode)
+    bce_loss(ref, torch.from_numpy(cw).double()).backward()
+    o, r = out.detach().cpu().double(), ref.detach()
+    assert ((o - r).abs() <= 3e-5 * r.abs().clamp_min(1.0)).all()
+    for g, gr in zip(p, p64):
+        rel = (g.grad.cpu().double() - gr.grad).abs().max() / gr.grad.abs().max()
+        assert float(rel) < 1e-3, rel

@@ -121,10 +121,11 @@ class WeightedMinSum:
                 llr = llr.contiguous()
                 a = alpha.detach().contiguous().float()
                 b = beta.detach().contiguous().float()
-                rec = torch.empty((iters, code.nc, nblk, 16), dtype=torch.uint8,
+                nbp = (nblk + 3) // 4 * 4       # the kernels' blocks, padded
+                rec = torch.empty((iters, code.nc, nbp, 16), dtype=torch.uint8,
                                   device=llr.device)
                 out = torch.empty_like(llr)
-                work = torch.empty(nblk * (2 * code.n + code.ne),
+                work = torch.empty(nbp * (2 * code.n + code.ne),
                                    dtype=torch.float32, device=llr.device)
                 N.call("atsc3_wms_forward_work", *code.ptrs(_CSR), code.n,
                        code.nc, code.ne, code.nbucket, nblk, iters,
@@ -144,7 +145,8 @@ class WeightedMinSum:
                 gt = g.contiguous().float()
                 ga = torch.zeros_like(a)
                 gb = torch.zeros_like(b)
-                work = torch.empty(nblk * code.n + 2 * nblk * code.ne,
+                nbp = rec.shape[2]
+                work = torch.empty(nbp * (code.n + 2 * code.ne),
                                    dtype=torch.float32, device=llr.device)
                 N.call("atsc3_wms_gradients", *code.ptrs(_CSR), code.n, code.nc,
                        code.ne, code.nbucket, nblk, iters,

@@ -355,8 +355,8 @@ int32_t atsc3_ldpc_qce_decode_weighted_rows(
  * (lab/m3_ldpc.py:459-482 layout); llr (nblk, ld_llr) float64; bits (nblk,
  * ld_bits) uint8; conv/its/bad per block; work: atsc3_ldpc_sp_workspace
  * bytes, 8-byte aligned.  atsc3_ldpc_sp_decode runs to `iters`: it
- * launches 4*(iters+1)+1 kernels on `stream` and returns without
- * synchronising.  atsc3_ldpc_sp_step runs ONE iteration `it` (it = 0
+ * launches one cooperative kernel per 256 codewords on `stream` and returns
+ * without synchronising.  atsc3_ldpc_sp_step runs ONE iteration `it` (it = 0
  * initialises the work area first; steps run in order on one stream),
  * so a host can honour the reference's wall-clock deadline between
  * iterations (lab/m16_margin.py:364-371): `last` = 1 takes the syndrome at

@@ -72,13 +72,14 @@ _QCE = {}
 
 def qce_plan(rate, n, cluster=0):
     """The edge-buffer quasi-cyclic plan of a code (every A/322 code) at a
-    cluster size (0: the smallest that holds a codeword), or None if that
-    decoder does not take it at that size."""
+    cluster size (0: the smallest that holds a codeword, for every batch: the
+    groups share the GPU), or None if that decoder does not take it at that
+    size."""
     key = (rate, n, cluster)
     if key not in _QCE:
         p = None
         try:
-            p = LDPC.QcePlan(rate, n, cluster=cluster)
+            p = LDPC.QcePlan(rate, n, cluster=cluster, wide=False)
         except N.FecError as e:
             if e.rc != -4:
                 raise

@@ -875,8 +875,9 @@ int32_t minsum_f32_host(const float *llr, int32_t nblk, int32_t n, int32_t nc,
     int32_t kq[3] = {0, 0, 0};
     if (atsc3_ldpc_qc_detect2(cptr, cidx, vptr, vedge, n, nc, nedges, kq,
                               rowptr.data(), addr.data()) == 0) {
-      const int32_t rc = atsc3_ldpc_qce_plan_create2(n, kq[0], kq[1], kq[2], rowptr.data(),
-                                                     addr.data(), 0, &qce);
+      // one cluster size: the callers of this entry decode from several threads
+      const int32_t rc = atsc3_ldpc_qce_plan_create_one(n, kq[0], kq[1], kq[2], rowptr.data(),
+                                                        addr.data(), &qce);
       if (rc != 0 && rc != -4) return rc;   // -4: a structure it does not take
       if (rc) qce = nullptr;
     }

@@ -98,6 +98,7 @@ struct QcePlan {
   int vbin_lo = 0, vbin_hi = 0; // least / most loaded variable-item bin (estimated cost)
   int ib[EMAXCL + 1] = {0};     // variable-phase items of CTA c in d_itab
   int cb[EMAXCL + 1] = {0};     // CTA c owns columns ccols[cb[c] .. cb[c+1])
+  char *d_blob = nullptr;       // one allocation for the tables below
   int4 *d_rdesc = nullptr;      // per row edge slot
   int32_t *d_ccols = nullptr;   // (nb) columns grouped by owner CTA
   int4 *d_itab = nullptr;       // variable-phase items, grouped by CTA
@@ -1614,17 +1615,98 @@ static int32_t qce_max_clusters(QceFn fn, int cl, int smem, int threads, int dev
   return 0;
 }
 
+// Copies a plan's tables to the device, in one allocation.  The bits' first
+// slots (s0, s0b) do not depend on the cluster size: `like` lends its own.
+static cudaError_t qce_upload(QcePlan &p, const QceTables &t, const QcePlan *like) {
+  struct Part {
+    void **dst;
+    const void *src;
+    size_t bytes;
+  };
+  const Part parts[] = {
+      {(void **)&p.d_rdesc, t.rdesc.data(), t.rdesc.size() * 16},
+      {(void **)&p.d_rptr, t.rptr.data(), t.rptr.size() * 4},
+      {(void **)&p.d_cdesc, t.cdesc.data(), t.cdesc.size() * 16},
+      {(void **)&p.d_ccols, t.ccols.data(), t.ccols.size() * 4},
+      {(void **)&p.d_itab, t.itab.data(), t.itab.size() * 16},
+      {(void **)&p.d_wbin, t.wbin.data(), t.wbin.size() * 4},
+      {(void **)&p.d_hitems, t.hitems.data(), t.hitems.size() * sizeof(int16_t)},
+      {(void **)&p.d_s0, t.s0.data(), like ? 0 : t.s0.size()},
+      {(void **)&p.d_s0b, t.s0b.data(), like ? 0 : t.s0b.size()},
+  };
+  auto room = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  size_t total = 0;
+  for (const Part &q : parts) {
+    total += room(q.bytes);
+    p.table_bytes += (int64_t)q.bytes;
+  }
+  std::vector<char> host(total);
+  cudaError_t e = cudaMalloc((void **)&p.d_blob, total ? total : 16);
+  if (e != cudaSuccess) return e;
+  size_t at = 0;
+  for (const Part &q : parts) {
+    if (q.bytes) std::memcpy(host.data() + at, q.src, q.bytes);
+    *q.dst = p.d_blob + at;
+    at += room(q.bytes);
+  }
+  if (like) {
+    p.d_s0 = like->d_s0;
+    p.d_s0b = like->d_s0b;
+  }
+  return total ? cudaMemcpy(p.d_blob, host.data(), total, cudaMemcpyHostToDevice) : cudaSuccess;
+}
+
 }  // namespace atsc3
 
 struct atsc3_ldpc_qce_plan {
   atsc3::QcePlan p;
+  // larger cluster sizes of the same code, for batches that leave SMs idle
+  std::vector<atsc3::QcePlan> wide;
 };
+
+namespace atsc3 {
+
+// Cluster sizes beside the plan's own, for batches with fewer codewords than
+// clusters of that size fit the chip: a codeword over more SMs takes fewer
+// items a warp in both phases.  (us an iteration, one codeword: 64800 6/15 with
+// 6 / 9 / 14 CTAs 15.7 / 13.3 / 10.9, 64800 13/15 with 6 / 12 20.2 / 13.3, 16200
+// 11/15 with 2 / 6 / 14 11.4 / 6.3 / 5.1, 16200 6/15 10.6 / 6.7 / 6.7.)
+constexpr int QCE_WIDE[] = {2, 3, 4, 6, 9, 10, 14};
+
+// The largest of them that holds all nblk codewords at once, else the plan's
+// own: with several rounds the SM time per codeword counts, and that grows with
+// the cluster (45 blocks of 64800 8/15 ending after 10 to 50 iterations: 1032 us
+// in rounds of 22 clusters of 6, 1047 in rounds of 15 of 9).  7 blocks of 64800
+// 10/15: 374 -> 280 us a decode chain, one of 16200 11/15 171 -> 89.
+static int32_t qce_choose(const atsc3_ldpc_qce_plan *h, int nblk, QceFn fn, int threads,
+                          const QcePlan **pick, int *ncl) {
+  int32_t rc = qce_max_clusters(fn, h->p.cluster, h->p.smem, threads, h->p.device, ncl);
+  if (rc) return rc;
+  *pick = &h->p;
+  for (const QcePlan &w : h->wide) {               // ascending sizes
+    int n = 0;
+    rc = qce_max_clusters(fn, w.cluster, w.smem, threads, w.device, &n);
+    if (rc) return rc;
+    if (n >= nblk) {
+      *pick = &w;
+      *ncl = n;
+    }
+  }
+  if (*ncl <= 0) {
+    set_error("unsupported: cluster configuration cannot be resident");
+    return -4;
+  }
+  return 0;
+}
+
+}  // namespace atsc3
 
 extern "C" {
 
 static int32_t qce_plan_create_vb(int32_t n, int32_t kldpc, int32_t qa, int32_t qb,
                                   const int32_t *rowptr, const int32_t *addr,
-                                  int32_t cluster, int vb, atsc3_ldpc_qce_plan **out) {
+                                  int32_t cluster, int vb, bool wide,
+                                  atsc3_ldpc_qce_plan **out) {
   using namespace atsc3;
   ATSC3_ARG(out && rowptr && addr, "null argument");
   *out = nullptr;
@@ -1689,22 +1771,17 @@ static int32_t qce_plan_create_vb(int32_t n, int32_t kldpc, int32_t qa, int32_t 
     return rc;
   }
   h->p.device = dev;
-  auto up = [&](void **dst, const void *src, size_t bytes) -> cudaError_t {
-    cudaError_t e = cudaMalloc(dst, bytes ? bytes : 16);
-    if (e != cudaSuccess) return e;
-    h->p.table_bytes += (int64_t)bytes;
-    return bytes ? cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice) : cudaSuccess;
-  };
-  cudaError_t e = up((void **)&h->p.d_rdesc, t.rdesc.data(), t.rdesc.size() * 16);
-  if (e == cudaSuccess) e = up((void **)&h->p.d_rptr, t.rptr.data(), t.rptr.size() * 4);
-  if (e == cudaSuccess) e = up((void **)&h->p.d_cdesc, t.cdesc.data(), t.cdesc.size() * 16);
-  if (e == cudaSuccess) e = up((void **)&h->p.d_ccols, t.ccols.data(), t.ccols.size() * 4);
-  if (e == cudaSuccess) e = up((void **)&h->p.d_itab, t.itab.data(), t.itab.size() * 16);
-  if (e == cudaSuccess) e = up((void **)&h->p.d_wbin, t.wbin.data(), t.wbin.size() * 4);
-  if (e == cudaSuccess) e = up((void **)&h->p.d_s0, t.s0.data(), t.s0.size());
-  if (e == cudaSuccess) e = up((void **)&h->p.d_s0b, t.s0b.data(), t.s0b.size());
-  if (e == cudaSuccess)
-    e = up((void **)&h->p.d_hitems, t.hitems.data(), t.hitems.size() * sizeof(int16_t));
+  cudaError_t e = qce_upload(h->p, t, nullptr);
+  if (wide)
+    for (int cl : QCE_WIDE) {
+      if (e != cudaSuccess || cl <= h->p.cluster) continue;
+      QcePlan w;
+      QceTables wt;
+      if (qce_build(n, kldpc, qa, qb, rowptr, addr, cl, &w, &wt, vb) || w.smem > smax) continue;
+      w.device = dev;
+      e = qce_upload(w, wt, &h->p);
+      h->wide.push_back(w);
+    }
   if (e != cudaSuccess) {
     atsc3_ldpc_qce_plan_destroy(h);
     return cuda_fail(e, "qce plan upload");
@@ -1717,14 +1794,21 @@ int32_t atsc3_ldpc_qce_plan_create2(int32_t n, int32_t kldpc, int32_t qa,
                                     int32_t qb, const int32_t *rowptr,
                                     const int32_t *addr, int32_t cluster,
                                     atsc3_ldpc_qce_plan **out) {
-  return qce_plan_create_vb(n, kldpc, qa, qb, rowptr, addr, cluster, 4, out);
+  return qce_plan_create_vb(n, kldpc, qa, qb, rowptr, addr, cluster, 4, cluster == 0, out);
+}
+
+int32_t atsc3_ldpc_qce_plan_create_one(int32_t n, int32_t kldpc, int32_t qa,
+                                       int32_t qb, const int32_t *rowptr,
+                                       const int32_t *addr,
+                                       atsc3_ldpc_qce_plan **out) {
+  return qce_plan_create_vb(n, kldpc, qa, qb, rowptr, addr, 0, 4, false, out);
 }
 
 int32_t atsc3_ldpc_qce_plan_create_f64(int32_t n, int32_t kldpc, int32_t qa,
                                        int32_t qb, const int32_t *rowptr,
                                        const int32_t *addr, int32_t cluster,
                                        atsc3_ldpc_qce_plan **out) {
-  return qce_plan_create_vb(n, kldpc, qa, qb, rowptr, addr, cluster, 8, out);
+  return qce_plan_create_vb(n, kldpc, qa, qb, rowptr, addr, cluster, 8, cluster == 0, out);
 }
 
 int32_t atsc3_ldpc_qce_plan_create(int32_t n, int32_t kldpc, int32_t qldpc,
@@ -1735,15 +1819,8 @@ int32_t atsc3_ldpc_qce_plan_create(int32_t n, int32_t kldpc, int32_t qldpc,
 
 void atsc3_ldpc_qce_plan_destroy(atsc3_ldpc_qce_plan *h) {
   if (!h) return;
-  cudaFree(h->p.d_rdesc);
-  cudaFree(h->p.d_rptr);
-  cudaFree(h->p.d_cdesc);
-  cudaFree(h->p.d_ccols);
-  cudaFree(h->p.d_itab);
-  cudaFree(h->p.d_wbin);
-  cudaFree(h->p.d_s0);
-  cudaFree(h->p.d_s0b);
-  cudaFree(h->p.d_hitems);
+  cudaFree(h->p.d_blob);
+  for (atsc3::QcePlan &w : h->wide) cudaFree(w.d_blob);
   delete h;
 }
 
@@ -1996,35 +2073,32 @@ static int32_t qce_decode_impl(
     int32_t threads, void *stream, bool f64, int wrow = 0) {
   using namespace atsc3;
   ATSC3_ARG(h != nullptr, "null plan");
-  const QcePlan &p = h->p;
-  ATSC3_ARG(p.vb == (f64 ? 8 : 4),
+  ATSC3_ARG(h->p.vb == (f64 ? 8 : 4),
             f64 ? "not a float64 plan (atsc3_ldpc_qce_plan_create_f64)"
                 : "a float64 plan needs atsc3_ldpc_qce_decode_f64");
   ATSC3_ARG(!(f64 && walpha), "learned weights are float32 only");
   ATSC3_ARG(nblk >= 0 && iters >= 0, "negative size");
   ATSC3_ARG(semantics == 0 || semantics == 1, "semantics must be 0 or 1");
   ATSC3_ARG(!(semantics == 1 && iters == 0), "semantics 1 needs iters >= 1");
-  ATSC3_ARG(ld_llr >= p.n, "ld_llr < n");
-  ATSC3_ARG(bits == nullptr || ld_bits >= p.n, "ld_bits < n");
-  ATSC3_ARG(hard == nullptr || ld_hard >= (p.n + 7) / 8, "ld_hard < ceil(n/8)");
+  ATSC3_ARG(ld_llr >= h->p.n, "ld_llr < n");
+  ATSC3_ARG(bits == nullptr || ld_bits >= h->p.n, "ld_bits < n");
+  ATSC3_ARG(hard == nullptr || ld_hard >= (h->p.n + 7) / 8, "ld_hard < ceil(n/8)");
   if (nblk == 0) return 0;
   ATSC3_ARG(conv && its && bad, "null status output");
   ATSC3_ARG(llr != nullptr, "null llr");
-  if (threads <= 0) threads = qce_default_threads(p.dr_light);
+  if (threads <= 0) threads = qce_default_threads(h->p.dr_light);
   ATSC3_ARG(threads == 512 || threads == 1024, "threads must be 512 or 1024");
-  if (qce_ns(p.dr_light) > 17 || f64) threads = 512;   // only the 512-thread build
-  QceFn fn = qce_fn(semantics, p.dr_light, threads, p.qb > 0, f64);
+  if (qce_ns(h->p.dr_light) > 17 || f64) threads = 512;   // only the 512-thread build
+  QceFn fn = qce_fn(semantics, h->p.dr_light, threads, h->p.qb > 0, f64);
   if (!fn) {
     set_error("unsupported: block-row degree too high");
     return -4;
   }
+  const QcePlan *pick = nullptr;
   int ncl = 0;
-  int32_t rc = qce_max_clusters(fn, p.cluster, p.smem, threads, p.device, &ncl);
+  const int32_t rc = qce_choose(h, nblk, fn, threads, &pick, &ncl);
   if (rc) return rc;
-  if (ncl <= 0) {
-    set_error("unsupported: cluster configuration cannot be resident");
-    return -4;
-  }
+  const QcePlan &p = *pick;
   ncl = std::min(ncl, nblk);
   QceArgs a;
   std::memset(&a, 0, sizeof(a));

@@ -128,11 +128,13 @@ class QcePlan(QcPlan):
     column owner, no per-check records.  Serves every A/322 code (Type A and
     Type B, where QcPlan takes Type B codes with one circulant per block);
     same semantics and outputs; cluster 0 picks the smallest cluster that
-    holds a codeword."""
+    holds a codeword, with larger ones beside it that a decode of few
+    codewords uses (wide=False: not, for decodes that share the GPU)."""
 
     kind = "qce"
 
-    def __init__(self, rate=None, n=None, cluster=0, dtype="float32", tables=None):
+    def __init__(self, rate=None, n=None, cluster=0, dtype="float32", tables=None,
+                 wide=True):
         """rate, n: an A/322 code; or tables = (n, K, qa, qb, rowptr, addr)
         as atsc3_ldpc_qc_detect2 recovers them from CSR tables.  dtype
         float32 or float64 (the float64 build: 8-byte slots, float64
@@ -152,8 +154,12 @@ class QcePlan(QcPlan):
         h = ctypes.c_void_p()
         fn = ("atsc3_ldpc_qce_plan_create_f64" if dtype == "float64"
               else "atsc3_ldpc_qce_plan_create2")
-        N.call(fn, n, K, qa, qb, rowptr.ctypes.data, addr.ctypes.data, int(cluster),
-               ctypes.byref(h))
+        if cluster == 0 and not wide and dtype == "float32":
+            N.call("atsc3_ldpc_qce_plan_create_one", n, K, qa, qb,
+                   rowptr.ctypes.data, addr.ctypes.data, ctypes.byref(h))
+        else:
+            N.call(fn, n, K, qa, qb, rowptr.ctypes.data, addr.ctypes.data,
+                   int(cluster), ctypes.byref(h))
         self._h = h
         self.n, self.nc, self.dtype = n, n - K, dtype
         info = np.zeros(10, np.int64)

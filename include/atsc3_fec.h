@@ -211,6 +211,15 @@ int32_t atsc3_ldpc_qce_plan_create2(int32_t n, int32_t kldpc, int32_t qa,
                                     int32_t qb, const int32_t *rowptr,
                                     const int32_t *addr, int32_t cluster,
                                     atsc3_ldpc_qce_plan **out);
+/* Cluster size: `cluster` > 0 pins it.  0 takes the smallest that holds a
+ * codeword and, beside it, larger ones that a decode of few codewords uses (a
+ * codeword over more SMs: up to twice as fast alone, at more SM time per
+ * codeword).  Where several decodes share the GPU on other streams or threads,
+ * atsc3_ldpc_qce_plan_create_one keeps the smallest size for every batch. */
+int32_t atsc3_ldpc_qce_plan_create_one(int32_t n, int32_t kldpc, int32_t qa,
+                                       int32_t qb, const int32_t *rowptr,
+                                       const int32_t *addr,
+                                       atsc3_ldpc_qce_plan **plan);
 
 /* The float64 edge-buffer decoder (8-byte slots, float64 messages and
  * posteriors, 512 threads per CTA): the arithmetic of the float64 paths of

@@ -98,11 +98,14 @@ struct QcePlan {
   int vbin_lo = 0, vbin_hi = 0; // least / most loaded variable-item bin (estimated cost)
   int ib[EMAXCL + 1] = {0};     // variable-phase items of CTA c in d_itab
   int cb[EMAXCL + 1] = {0};     // CTA c owns columns ccols[cb[c] .. cb[c+1])
+  int xb[EMAXCL + 1] = {0};     // CTA c's entries of the spread columns' table
+  int xt_off = 0;               // shared-memory offset of that table
   char *d_blob = nullptr;       // one allocation for the tables below
   int4 *d_rdesc = nullptr;      // per row edge slot
   int32_t *d_ccols = nullptr;   // (nb) columns grouped by owner CTA
   int4 *d_itab = nullptr;       // variable-phase items, grouped by CTA
   int32_t *d_wbin = nullptr;    // (cluster, QBINS+1) bin offsets into each CTA's items
+  uint32_t *d_xtab = nullptr;   // per slot of a spread column: CTA << 20 | byte offset
   int32_t *d_rptr = nullptr;    // (Q+1)
   int4 *d_cdesc = nullptr;      // per column
   uint8_t *d_s0 = nullptr;      // (nb*360) rotation start (zone A / only zone)
@@ -118,6 +121,8 @@ struct QcePlan {
 // y = byte offset of the edge's circulant slot in the owner's shared memory,
 // z = circulant shift u, w = byte offset of the column's bitmap words.
 // Check (r, k) reads entry (k - u) mod 360 of the slot.
+// (qce_spread then moves part of the slots from their column's CTA to their
+// row's; x and y name where they are.)
 // Column descriptor (column g): x = slots d, y = byte offset of slot 0 in
 // the owner's shared memory (slots follow at 1440-byte steps, sorted by
 // (zone, u, row)), z = index of the dual-diagonal wrap slot (absent for bit
@@ -130,6 +135,7 @@ struct QceTables {
   std::vector<int32_t> ccols;
   std::vector<int4> itab;
   std::vector<int32_t> wbin;    // (cluster, QBINS+1) bin offsets, relative to ib[c]
+  std::vector<uint32_t> xtab;   // spread columns' slots, grouped by CTA
   std::vector<uint8_t> s0, s0b;
   std::vector<int16_t> hitems;
 };
@@ -140,6 +146,45 @@ constexpr int VM_EXACT = 1;    // 1..4 slots of one zone, rotated in registers
 constexpr int VM_GEN = 2;      // any slots of one zone, rotated by offsets
 constexpr int VM_GEN2 = 3;     // slots in both zones: two rotated segments
 constexpr uint32_t VNOWRAP = 0xFFu;
+constexpr int VSPREAD = 1 << 27;   // of z: the slots' addresses are in the spread table
+                                   // (x = first entry | first bit of the item << 16)
+
+// Deals a CTA's variable-phase items to QBINS bins, the most expensive first,
+// each to the least-loaded bin (longest-processing-time rule), so that every
+// warp walking its own bin has about the same work; a bin keeps its items in
+// column order.  Estimated cost (cycles per item of a 1024-thread CTA under full
+// load, fitted to per-warp phase times of 64800-bit 6/15, 8/15 and 10/15
+// codewords): pair 840, 1-4 slots in registers 280 + 240 d (spread: + 60 d), any
+// slots 1330 + 140 d (two zones: + 200).
+static void qce_deal(const std::vector<int4> &items, int c, QcePlan *p, QceTables *t) {
+  std::vector<int> cost(items.size()), order(items.size());
+  for (size_t i = 0; i < items.size(); ++i) {
+    const int d = items[i].z & 0xFF, mode = (items[i].z >> 25) & 3;
+    cost[i] = mode == VM_PAIR ? 840 : mode == VM_EXACT ? 280 + 240 * d
+            : mode == VM_GEN ? 1330 + 140 * d : 1530 + 140 * d;
+    if (items[i].z & VSPREAD) cost[i] += 60 * d;
+    order[i] = (int)i;
+  }
+  std::stable_sort(order.begin(), order.end(),
+                   [&](int x, int y) { return cost[x] > cost[y]; });
+  std::vector<std::vector<int>> bins(QBINS);
+  std::vector<int> load(QBINS, 0);
+  for (int i : order) {
+    const int b = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+    bins[b].push_back(i);
+    load[b] += cost[i];
+  }
+  const int first = (int)t->itab.size();
+  for (int b = 0; b < QBINS; ++b) {
+    std::sort(bins[b].begin(), bins[b].end());
+    t->wbin[(size_t)c * (QBINS + 1) + b] = (int)t->itab.size() - first;
+    for (int i : bins[b]) t->itab.push_back(items[i]);
+    p->vbin_lo = std::min(p->vbin_lo, load[b]);
+    p->vbin_hi = std::max(p->vbin_hi, load[b]);
+  }
+  t->wbin[(size_t)c * (QBINS + 1) + QBINS] = (int)t->itab.size() - first;
+  p->ib[c + 1] = (int)t->itab.size();
+}
 
 int qce_build(int n, int K, int QA, int QB, const int32_t *rowptr,
               const int32_t *addr, int cluster, QcePlan *p, QceTables *t,
@@ -528,42 +573,169 @@ int qce_build(int n, int K, int QA, int QB, const int32_t *rowptr,
                                   (int)w));
       }
     }
-    // Deal the CTA's items to QBINS bins, the most expensive first, each to
-    // the least-loaded bin (longest-processing-time rule), so that every
-    // warp walking its own bin has about the same work; a bin keeps its
-    // items in column order.  Estimated cost (cycles per item of a
-    // 1024-thread CTA under full load, fitted to per-warp phase times of
-    // 64800-bit 6/15, 8/15 and 10/15 codewords): pair 840, 1-4 slots in
-    // registers 280 + 240 d, any slots 1330 + 140 d (two zones: + 200).
-    std::vector<int> cost(items.size()), order(items.size());
-    for (size_t i = 0; i < items.size(); ++i) {
-      const int d = items[i].z & 0xFF, mode = (items[i].z >> 25) & 3;
-      cost[i] = mode == VM_PAIR ? 840 : mode == VM_EXACT ? 280 + 240 * d
-              : mode == VM_GEN ? 1330 + 140 * d : 1530 + 140 * d;
-      order[i] = (int)i;
-    }
-    std::stable_sort(order.begin(), order.end(),
-                     [&](int x, int y) { return cost[x] > cost[y]; });
-    std::vector<std::vector<int>> bins(QBINS);
-    std::vector<int> load(QBINS, 0);
-    for (int i : order) {
-      const int b = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-      bins[b].push_back(i);
-      load[b] += cost[i];
-    }
-    const int first = (int)t->itab.size();
-    for (int b = 0; b < QBINS; ++b) {
-      std::sort(bins[b].begin(), bins[b].end());
-      t->wbin[(size_t)c * (QBINS + 1) + b] = (int)t->itab.size() - first;
-      for (int i : bins[b]) t->itab.push_back(items[i]);
-      p->vbin_lo = std::min(p->vbin_lo, load[b]);
-      p->vbin_hi = std::max(p->vbin_hi, load[b]);
-    }
-    t->wbin[(size_t)c * (QBINS + 1) + QBINS] = (int)t->itab.size() - first;
-    p->ib[c + 1] = (int)t->itab.size();
+    qce_deal(items, c, p, t);
   }
   for (int c = cluster + 1; c <= EMAXCL; ++c) p->ib[c] = p->ib[cluster];
   return 0;
+}
+
+// Moves part of the slots of short information columns from their column's CTA to
+// the CTA that owns their row.  A slot at its column costs the check phase one
+// remote load and one remote store an entry, a slot at its row costs them to the
+// variable phase.  With every slot at its column the check phase is bound by the
+// distributed shared memory (a warp's load and store of 32 entries take 18 to 24
+// cycles of an SM's share; 64800 6/15 on 6 CTAs: 828 of them, 18.3k of an
+// iteration's 32.8k cycles) while the variable phase leaves it idle.  Columns of
+// up to 4 edges are the ones to move: their items hold all their slots in
+// registers, so each is still read once (a longer column's item reads them twice
+// and becomes the phase's longest: 64800 6/15 413 us without, 456 with one such
+// column, 594 with all 13).
+// Each move is the one that relieves the busiest CTAs most; it is not made where
+// the variable phase would then carry more than `share` of what the check phase
+// still does, nor into a CTA whose shared memory (smax bytes) is full.  Half is
+// best up to 6 CTAs, a quarter beyond, where a warp has one or two items a phase
+// and the remote loads' latency shows.  24 iterations, us, none moved / moved:
+// 64800 on 6 CTAs, 22 codewords: 6/15 449 / 398, 8/15 458 / 417, 9/15 470 / 415,
+// 10/15 463 / 439, 11/15 478 / 431, 12/15 526 / 475, 13/15 535 / 491; 8/15 on 9
+// CTAs 399 / 369, 10/15 on 14 CTAs 316 / 295; 16200 8/15 on 6 CTAs 214 / 197; on
+// 2 CTAs nothing is gained (290 / 292, 304 / 310, 402 / 400).
+static void qce_spread(QcePlan *p, QceTables *t, int smax) {
+  const int cl = p->cluster, slotb = EZ * p->vb, Q = p->Q, nbi = p->K / EZ;
+  if (cl < 3) return;
+  // the CTA that owns a light row (a Type A code's ranges may split a row: its
+  // first chunk's CTA); heavy rows are shared by all
+  std::vector<int> rowown(Q, -1);
+  for (int c = 0; c < cl; ++c)
+    for (int i = p->ci[c]; i < p->ci[c + 1]; ++i)
+      if (rowown[i / ECHUNK] < 0) rowown[i / ECHUNK] = c;
+  // candidates: information columns of register items (VM_EXACT)
+  std::vector<int> mode(p->nb, VM_PAIR);
+  for (const int4 &v : t->itab) mode[v.y / EZ] = (v.z >> 25) & 3;
+  struct Move {
+    int rd, from, to;            // row slot, CTAs
+  };
+  std::vector<int> load(cl, 0);          // places taken
+  for (int g = 0; g < p->nb; ++g) load[t->cdesc[g].w & 0xFF] += t->cdesc[g].x;
+  const std::vector<int> used(load);
+  // remote slots a CTA reaches or serves: in the check phase, and in the variable
+  // phase for the moved ones
+  std::vector<int> lc(cl, 0), lv(cl, 0);
+  std::vector<Move> open, moves;
+  std::vector<char> isx(p->nb, 0);
+  for (int r = 0; r < Q; ++r)
+    for (int e = t->rptr[r]; e < t->rptr[r + 1]; ++e) {
+      const int g = t->rdesc[e].w / (ECHUNK * 4), own = t->rdesc[e].x & 0xFF;
+      if (rowown[r] < 0 || own == rowown[r]) continue;
+      ++lc[own];
+      ++lc[rowown[r]];
+      if (g < nbi && mode[g] == VM_EXACT) {
+        open.push_back(Move{e, own, rowown[r]});
+        isx[g] = 1;
+      }
+    }
+  // the table takes at most a word per slot
+  const int cap = (smax - p->buf_off - 4 * p->max_slots - 16) / slotb;
+  if (cap < p->max_slots) return;
+  const double share = cl <= 6 ? 0.5 : 0.25;
+  while (!open.empty()) {
+    int best = -1;
+    double bs = 0.0;
+    for (size_t i = 0; i < open.size(); ++i) {
+      const Move &m = open[i];
+      if (load[m.to] >= cap) continue;
+      if (std::max(lv[m.from], lv[m.to]) + 1 > share * std::max(lc[m.from], lc[m.to])) continue;
+      const double sc = (double)lc[m.from] * lc[m.from] + (double)lc[m.to] * lc[m.to] -
+                        0.5 * ((double)lv[m.from] * lv[m.from] + (double)lv[m.to] * lv[m.to]) +
+                        1e-3 * (load[m.from] - load[m.to]) + 1e6;
+      if (best < 0 || sc > bs) {
+        best = (int)i;
+        bs = sc;
+      }
+    }
+    if (best < 0) break;
+    const Move m = open[best];
+    moves.push_back(m);
+    open.erase(open.begin() + best);
+    --lc[m.from];
+    --lc[m.to];
+    ++lv[m.from];
+    ++lv[m.to];
+    --load[m.from];
+    ++load[m.to];
+  }
+  // free places: the moved slots' own, then the space past the CTA's columns
+  std::vector<std::vector<int>> holes(cl);
+  for (int c = 0; c < cl; ++c)
+    for (int q = cap; q-- > used[c];) holes[c].push_back(p->buf_off + q * slotb);
+  for (const Move &m : moves) holes[m.from].push_back(t->rdesc[m.rd].y);
+  int top = p->buf_off + p->max_slots * slotb;       // end of the space used
+  std::vector<char> spread(p->nb, 0);
+  // where every slot of a candidate column lives: (CTA, byte offset)
+  std::vector<std::vector<uint32_t>> at(p->nb);
+  for (int g = 0; g < nbi; ++g)
+    if (isx[g])
+      for (int i = 0; i < t->cdesc[g].x; ++i)
+        at[g].push_back((uint32_t)(t->cdesc[g].w & 0xFF) << 20 | (uint32_t)(t->cdesc[g].y + i * slotb));
+  for (const Move &m : moves) {
+    int4 &d = t->rdesc[m.rd];
+    const int g = d.w / (ECHUNK * 4), i = (d.y - t->cdesc[g].y) / slotb;
+    spread[g] = 1;
+    at[g][i] = (uint32_t)m.to << 20 | (uint32_t)holes[m.to].back();
+    top = std::max(top, holes[m.to].back() + slotb);
+    holes[m.to].pop_back();
+  }
+  for (const Move &m : moves) {
+    int4 &d = t->rdesc[m.rd];
+    const int g = d.w / (ECHUNK * 4), i = (d.y - t->cdesc[g].y) / slotb;
+    d.x = (d.x & ~0xFF) | (int)(at[g][i] >> 20);
+    d.y = (int)(at[g][i] & 0xFFFFF);
+  }
+  // the table: per CTA, its spread columns' slots
+  t->xtab.clear();
+  std::vector<int> first(p->nb, 0);
+  int most = 0;
+  for (int c = 0; c < cl; ++c) {
+    p->xb[c] = (int)t->xtab.size();
+    for (int q = p->cb[c]; q < p->cb[c + 1]; ++q) {
+      const int g = t->ccols[q];
+      if (!spread[g]) continue;
+      first[g] = (int)t->xtab.size() - p->xb[c];
+      t->xtab.insert(t->xtab.end(), at[g].begin(), at[g].end());
+    }
+    most = std::max(most, (int)t->xtab.size() - p->xb[c]);
+  }
+  for (int c = cl; c <= EMAXCL; ++c) p->xb[c] = (int)t->xtab.size();
+  // the slots move up by the table's size
+  const int grow = (most * 4 + 15) & ~15;
+  p->xt_off = p->buf_off;
+  p->max_slots = (top - p->buf_off) / slotb;
+  p->buf_off += grow;
+  p->smem = top + grow;
+  for (int4 &d : t->rdesc) d.y += grow;
+  for (int4 &d : t->cdesc) d.y += grow;
+  for (uint32_t &x : t->xtab) x += (uint32_t)grow;
+  QceTables old;
+  old.itab.swap(t->itab);
+  int ib[EMAXCL + 1];
+  std::copy(p->ib, p->ib + EMAXCL + 1, ib);
+  p->vbin_lo = 1 << 30;
+  p->vbin_hi = 0;
+  for (int c = 0; c < cl; ++c) {
+    std::vector<int4> items(old.itab.begin() + ib[c], old.itab.begin() + ib[c + 1]);
+    for (int4 &v : items) {
+      const int g = v.y / EZ;
+      if (spread[g]) {
+        v.x = first[g] | (v.y - g * EZ) << 16;
+        v.z |= VSPREAD;
+      } else {
+        v.x += grow;
+      }
+    }
+    std::stable_sort(items.begin(), items.end(),
+                     [](const int4 &a, const int4 &b) { return a.y < b.y; });
+    qce_deal(items, c, p, t);
+  }
+  for (int c = cl + 1; c <= EMAXCL; ++c) p->ib[c] = p->ib[cl];
 }
 
 struct QceArgs {
@@ -575,8 +747,9 @@ struct QceArgs {
   // shared-memory layout (byte offsets): syndrome exchange words, per-chunk
   // row-slot table, per-row info, variable-phase items, heavy-row slots; the
   // bitmap sits at 0
-  int part_off, rt_off, ri_off, ct_off, ht_off;
+  int part_off, rt_off, ri_off, ct_off, ht_off, xt_off;
   int ci[EMAXCL + 1];
+  int xb[EMAXCL + 1];
   int cb[EMAXCL + 1];
   int ib[EMAXCL + 1];
   int hoff[EMAXCL + 1];         // heavy items of CTA c: hitems[hoff[c] .. hoff[c+1])
@@ -586,6 +759,7 @@ struct QceArgs {
   const int32_t *ccols;
   const int4 *itab;
   const int32_t *wbin;          // (cluster, QBINS+1) item-bin offsets per CTA
+  const uint32_t *xtab;         // spread columns' slots: CTA << 20 | byte offset
   const int4 *rdesc;
   const int32_t *rptr;
   const int4 *cdesc;
@@ -638,6 +812,43 @@ __device__ __forceinline__ V qce_var_exact(V *col, int s0, V li, bool mv) {
 }
 
 
+
+// The same for the two bits a lane takes of a spread column: slot i of the column
+// is at cluster address tab[i], in whichever CTA (qce_spread).  All loads are
+// issued before the first sum.
+template <typename V, bool TORCH, int D>
+__device__ __forceinline__ void qce_var_spread(const uint32_t *tab, uint32_t off0, uint32_t off1,
+                                               int s00, int s01, V li0, V li1, bool mv0, bool mv1,
+                                               V &t0, V &t1) {
+  uint32_t ad[D];
+  V m0[D], m1[D];
+#pragma unroll
+  for (int i = 0; i < D; ++i) {
+    ad[i] = tab[i];
+    m0[i] = dsmem_ld<V>(ad[i] + off0);
+    m1[i] = dsmem_ld<V>(ad[i] + off1);
+  }
+  const int r0 = s00 >= D ? s00 - D : s00, r1 = s01 >= D ? s01 - D : s01;
+  V a0 = TORCH ? li0 : V(0), a1 = TORCH ? li1 : V(0);
+#pragma unroll
+  for (int t = 0; t < D; ++t) {
+    V v0 = m0[t], v1 = m1[t];
+#pragma unroll
+    for (int c = 1; c < D; ++c) {
+      v0 = (r0 == c) ? m0[(c + t) % D] : v0;
+      v1 = (r1 == c) ? m1[(c + t) % D] : v1;
+    }
+    a0 = add_rn(a0, v0);
+    a1 = add_rn(a1, v1);
+  }
+  t0 = TORCH ? add_rn(a0, V(0)) : add_rn(li0, a0);     // no -0.0 (see qce_var_exact)
+  t1 = TORCH ? add_rn(a1, V(0)) : add_rn(li1, a1);
+#pragma unroll
+  for (int i = 0; i < D; ++i) {
+    if (mv0) dsmem_st_bits(ad[i] + off0, vbits(sub_rn(t0, m0[i])));
+    if (mv1) dsmem_st_bits(ad[i] + off1, vbits(sub_rn(t1, m1[i])));
+  }
+}
 
 // Sums of one zone's slots of a column (`c0`, `c1` = the first slot of the
 // two bits a lane takes in a 64-bit item, d slots) in each bit's reference
@@ -1200,6 +1411,12 @@ __global__ void __launch_bounds__(NT, 1) ldpc_qce_kernel(const QceArgs a) {
     const int4 v = __ldg(a.itab + i0 + q);
     itab[q] = make_uint4((uint32_t)v.x, (uint32_t)v.y, (uint32_t)v.z, (uint32_t)v.w);
   }
+  // the spread columns' slots: cluster address of each
+  uint32_t *xtab = reinterpret_cast<uint32_t *>(smem + a.xt_off);
+  for (int q = tid; q < a.xb[rank + 1] - a.xb[rank]; q += blockDim.x) {
+    const uint32_t v = __ldg(a.xtab + a.xb[rank] + q);
+    xtab[q] = dsmem_map(sm_sa + (v & 0xFFFFFu), v >> 20);
+  }
   if (tid == 0) {
     part[0] = 0;
     part[1] = 0;
@@ -1239,12 +1456,17 @@ __global__ void __launch_bounds__(NT, 1) ldpc_qce_kernel(const QceArgs a) {
         const bool mv = (uint32_t)lane < nval;
         const bool absent = sub == asub && ((iw.z >> 24) & 1u) && lane == ABSENT_LANE;
         const V li = mv ? lam[iw.y + 32 * sub + lane] : V(0);
-        V *col = reinterpret_cast<V *>(smem + iw.x) + 32 * sub + lane;
         // q = lam - 0; stored as lam + 0 (+0.0 for a -0.0 LLR, which the
         // check phase's sign-bit tests then read like the reference's v < 0)
         const V lq = add_rn(li, V(0));
-        if (mv)
+        if (iw.z & (uint32_t)VSPREAD) {
+          const uint32_t off = (uint32_t)sizeof(V) * ((iw.x >> 16) + 32u * sub + lane);
+          if (mv)
+            for (int i = 0; i < d; ++i) dsmem_st_bits(xtab[(iw.x & 0xFFFFu) + i] + off, vbits(lq));
+        } else if (mv) {
+          V *col = reinterpret_cast<V *>(smem + iw.x) + 32 * sub + lane;
           for (int i = 0; i < d; ++i) col[i * EZ] = (absent && i == wrapi) ? V(-0.0) : lq;
+        }
         const uint32_t hb = __ballot_sync(0xffffffffu, mv && li < V(0));
         if (lane < CL) dsmem_st_u32(bm_peer + ((iw.w & 0xFFFFu) + sub) * 4u, hb);
       }
@@ -1433,7 +1655,19 @@ __global__ void __launch_bounds__(NT, 1) ldpc_qce_kernel(const QceArgs a) {
           V *col0 = reinterpret_cast<V *>(smem + iw.x) + l0;
           V *col1 = reinterpret_cast<V *>(smem + iw.x) + l1;
           V t0, t1;
-          if (mode == VM_PAIR) {
+          if (iw.z & (uint32_t)VSPREAD) {
+            const uint32_t *tab = xtab + (iw.x & 0xFFFFu);
+            const uint32_t off0 = (uint32_t)sizeof(V) * ((iw.x >> 16) + (uint32_t)l0);
+            const uint32_t off1 = (uint32_t)sizeof(V) * ((iw.x >> 16) + (uint32_t)l1);
+            if (d == 3)
+              qce_var_spread<V, TORCH, 3>(tab, off0, off1, cur.s00, cur.s01, li0, li1, mv0, mv1, t0, t1);
+            else if (d == 4)
+              qce_var_spread<V, TORCH, 4>(tab, off0, off1, cur.s00, cur.s01, li0, li1, mv0, mv1, t0, t1);
+            else if (d == 2)
+              qce_var_spread<V, TORCH, 2>(tab, off0, off1, cur.s00, cur.s01, li0, li1, mv0, mv1, t0, t1);
+            else
+              qce_var_spread<V, TORCH, 1>(tab, off0, off1, cur.s00, cur.s01, li0, li1, mv0, mv1, t0, t1);
+          } else if (mode == VM_PAIR) {
             // dual-diagonal parity column: slots in check order for every
             // bit (u = 0 twice, or u = 0, 1 for the last column, whose wrap
             // entry of bit 359 is absent and holds -0.0)
@@ -1630,6 +1864,7 @@ static cudaError_t qce_upload(QcePlan &p, const QceTables &t, const QcePlan *lik
       {(void **)&p.d_ccols, t.ccols.data(), t.ccols.size() * 4},
       {(void **)&p.d_itab, t.itab.data(), t.itab.size() * 16},
       {(void **)&p.d_wbin, t.wbin.data(), t.wbin.size() * 4},
+      {(void **)&p.d_xtab, t.xtab.data(), t.xtab.size() * 4},
       {(void **)&p.d_hitems, t.hitems.data(), t.hitems.size() * sizeof(int16_t)},
       {(void **)&p.d_s0, t.s0.data(), like ? 0 : t.s0.size()},
       {(void **)&p.d_s0b, t.s0b.data(), like ? 0 : t.s0b.size()},
@@ -1771,6 +2006,7 @@ static int32_t qce_plan_create_vb(int32_t n, int32_t kldpc, int32_t qa, int32_t 
     return rc;
   }
   h->p.device = dev;
+  qce_spread(&h->p, &t, smax);
   cudaError_t e = qce_upload(h->p, t, nullptr);
   if (wide)
     for (int cl : QCE_WIDE) {
@@ -1778,6 +2014,7 @@ static int32_t qce_plan_create_vb(int32_t n, int32_t kldpc, int32_t qa, int32_t 
       QcePlan w;
       QceTables wt;
       if (qce_build(n, kldpc, qa, qb, rowptr, addr, cl, &w, &wt, vb) || w.smem > smax) continue;
+      qce_spread(&w, &wt, smax);
       w.device = dev;
       e = qce_upload(w, wt, &h->p);
       h->wide.push_back(w);
@@ -1883,6 +2120,35 @@ int32_t atsc3_ldpc_qce_tables_host2(int32_t n, int32_t kldpc, int32_t qa,
   if (itab) std::memcpy(itab, t.itab.data(), t.itab.size() * 16);
   if (hitems)
     for (size_t i = 0; i < t.hitems.size(); ++i) hitems[i] = t.hitems[i];
+  return 0;
+}
+
+int32_t atsc3_ldpc_qce_spread_host(int32_t n, int32_t kldpc, int32_t qa, int32_t qb,
+                                   const int32_t *rowptr, const int32_t *addr,
+                                   int32_t cluster, int32_t smax, int32_t *meta,
+                                   int32_t *rdesc, int32_t *itab, int32_t *xtab) {
+  using namespace atsc3;
+  ATSC3_ARG(meta && rowptr && addr, "null argument");
+  QcePlan p;
+  QceTables t;
+  const int rc = qce_build(n, kldpc, qa, qb, rowptr, addr, cluster, &p, &t);
+  if (rc) return rc;
+  qce_spread(&p, &t, smax);
+  meta[0] = (int32_t)t.rdesc.size();
+  meta[1] = (int32_t)t.itab.size();
+  meta[2] = (int32_t)t.xtab.size();
+  meta[3] = p.smem;
+  meta[4] = p.buf_off;
+  meta[5] = p.xt_off;
+  meta[6] = p.max_slots;
+  for (int c = 0; c <= EMAXCL; ++c) {
+    meta[7 + c] = p.xb[c];
+    meta[24 + c] = p.ib[c];
+    meta[41 + c] = p.ci[c];
+  }
+  if (rdesc) std::memcpy(rdesc, t.rdesc.data(), t.rdesc.size() * 16);
+  if (itab) std::memcpy(itab, t.itab.data(), t.itab.size() * 16);
+  if (xtab) std::memcpy(xtab, t.xtab.data(), t.xtab.size() * 4);
   return 0;
 }
 
@@ -2114,10 +2380,12 @@ static int32_t qce_decode_impl(
   a.ri_off = p.ri_off;
   a.ct_off = p.ct_off;
   a.ht_off = p.ht_off;
+  a.xt_off = p.xt_off;
   for (int c = 0; c <= EMAXCL; ++c) {
     a.ci[c] = p.ci[c];
     a.cb[c] = p.cb[c];
     a.hoff[c] = p.hoff[c];
+    a.xb[c] = p.xb[c];
   }
   a.nhrows = p.nhrows;
   a.hsplit = p.hsplit;
@@ -2126,6 +2394,7 @@ static int32_t qce_decode_impl(
   a.ccols = p.d_ccols;
   a.itab = p.d_itab;
   a.wbin = p.d_wbin;
+  a.xtab = p.d_xtab;
   for (int c = 0; c <= EMAXCL; ++c) a.ib[c] = p.ib[c];
   a.rdesc = p.d_rdesc;
   a.rptr = p.d_rptr;

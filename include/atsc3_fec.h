@@ -319,6 +319,19 @@ int32_t atsc3_ldpc_qce_bins_host(int32_t n, int32_t kldpc, int32_t qa, int32_t q
                                  const int32_t *rowptr, const int32_t *addr,
                                  int32_t cluster, int32_t *wbin);
 
+/* Host only: the layout a plan decodes with, short columns' slots moved to their
+ * rows' CTAs (smax: shared memory of a CTA in bytes).  meta (58 ints): [0] row
+ * slots, [1] items, [2] entries of xtab, [3] shared memory per CTA, [4] offset of
+ * the slots, [5] of the table of moved columns, [6] slots per CTA, [7..23] first
+ * xtab entry, [24..40] first item, [41..57] first check item of each CTA.  rdesc
+ * and itab as atsc3_ldpc_qce_tables_host2; an item with bit 27 of z set names
+ * its slots in xtab (x = first entry | first bit << 16; an entry is CTA << 20 |
+ * byte offset). */
+int32_t atsc3_ldpc_qce_spread_host(int32_t n, int32_t kldpc, int32_t qa, int32_t qb,
+                                   const int32_t *rowptr, const int32_t *addr,
+                                   int32_t cluster, int32_t smax, int32_t *meta,
+                                   int32_t *rdesc, int32_t *itab, int32_t *xtab);
+
 int32_t atsc3_ldpc_qce_config(const atsc3_ldpc_qce_plan *plan, int32_t threads,
                               int32_t semantics, int32_t *out);
 

@@ -7,10 +7,16 @@
 // R[pos] = x^(K-1-pos) mod g(x) -- the same GF(2) matrix product
 // lab/m9_accel.py:169-236 evaluates with popcounts.  Zero syndrome = BCH OK.
 //
-// One CTA per codeword; each thread folds the rows of the bits it owns into
-// six 32-bit words, then a warp-shuffle and shared-memory XOR reduction.
+// A cluster of CTAs per codeword.  A warp folds the table rows of one 32-bit word
+// of decisions at a time, a row per lane (the word's 32 rows are 768 contiguous
+// bytes, those of clear bits predicated off) and eight words in flight; then a
+// warp XOR, a shared-memory XOR, and the first CTA adds the others' through
+// distributed shared memory.  The table sits in L2; with one CTA a codeword and a
+// word a thread, its latency and the 32 lines each load touched were the bound
+// (one 16200 11/15 codeword 13.3 us, 7 of 64800 10/15 37.8, 75 of 6/15 26.6; now
+// 3.6, 5.8 and 9.8).
 // The descrambled payload (lab/m9_fast.py:942-949: hard bits XOR the
-// scrambling sequence, packed MSB-first) is written by the same CTA.
+// scrambling sequence, packed MSB-first) is written by the same cluster.
 
 #include <cuda_runtime.h>
 
@@ -19,8 +25,10 @@
 
 namespace atsc3 {
 
-__device__ __forceinline__ void fold_row(uint32_t (&acc)[6],
-                                         const uint32_t *__restrict__ rtab,
+constexpr int BCH_T = 256;
+constexpr int BCH_CL = 8;             // CTAs per codeword at most (portable cluster)
+
+__device__ __forceinline__ void fold_row(uint32_t (&acc)[6], const uint32_t *__restrict__ rtab,
                                          int pos) {
   const uint2 *r = reinterpret_cast<const uint2 *>(rtab + (size_t)pos * 6);
   const uint2 a = __ldg(r), b = __ldg(r + 1), c = __ldg(r + 2);
@@ -28,13 +36,13 @@ __device__ __forceinline__ void fold_row(uint32_t (&acc)[6],
   acc[3] ^= b.y; acc[4] ^= c.x; acc[5] ^= c.y;
 }
 
-__device__ __forceinline__ void reduce_store(uint32_t (&acc)[6], uint32_t *syn,
-                                             uint8_t *ok) {
-  __shared__ uint32_t red[32][6];
+// The cluster's XOR of acc, written by its first CTA.
+__device__ __forceinline__ void reduce_store(uint32_t (&acc)[6], uint32_t *syn, uint8_t *ok) {
+  __shared__ uint32_t red[BCH_T / 32][6];
+  __shared__ uint32_t all[BCH_CL][6];           // rank 0: every CTA's words
+  const int rank = (int)cluster_ctarank(), cl = (int)cluster_nctarank();
 #pragma unroll
-  for (int w = 0; w < 6; ++w)
-    for (int o = 16; o > 0; o >>= 1)
-      acc[w] ^= __shfl_xor_sync(0xffffffffu, acc[w], o);
+  for (int w = 0; w < 6; ++w) acc[w] = __reduce_xor_sync(0xffffffffu, acc[w]);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (lane == 0)
 #pragma unroll
@@ -42,56 +50,111 @@ __device__ __forceinline__ void reduce_store(uint32_t (&acc)[6], uint32_t *syn,
   __syncthreads();
   if (threadIdx.x < 6) {
     uint32_t v = 0;
-    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) v ^= red[q][threadIdx.x];
-    syn[threadIdx.x] = v;
-    red[0][threadIdx.x] = v;   // safe: every warp's value already folded
+    for (int q = 0; q < BCH_T / 32; ++q) v ^= red[q][threadIdx.x];
+    dsmem_st_u32(dsmem_map(smem_u32(&all[rank][threadIdx.x]), 0u), v);
   }
-  __syncthreads();
-  if (threadIdx.x == 0 && ok) {
-    uint32_t any = 0;
-    for (int w = 0; w < 6; ++w) any |= red[0][w];
-    *ok = any == 0 ? 1 : 0;
+  cluster_sync_all();
+  if (rank == 0 && warp == 0) {
+    uint32_t v = 0;
+    if (lane < 6) {
+      for (int q = 0; q < cl; ++q) v ^= all[q][lane];
+      syn[lane] = v;
+    }
+    const bool any = __any_sync(0xffffffffu, v != 0);
+    if (lane == 0 && ok) *ok = any ? 0 : 1;
   }
 }
 
-__global__ void __launch_bounds__(256) bch_packed_kernel(
+// this warp's words of a packed codeword and this thread's share of the payload
+__device__ __forceinline__ void fold_packed(uint32_t (&acc)[6], const uint8_t *h, int kldpc,
+                                            const uint32_t *__restrict__ rtab,
+                                            const uint8_t *__restrict__ scr, int kpay,
+                                            uint8_t *__restrict__ po) {
+  const int t0 = (int)cluster_ctarank() * BCH_T + threadIdx.x;
+  const int step = (int)cluster_nctarank() * BCH_T;
+  const int nword = kldpc >> 5;              // whole 32-bit words
+  const uint32_t *hw = reinterpret_cast<const uint32_t *>(h);
+  const int lane = threadIdx.x & 31;
+  // row 32w + l of word w is decided by bit l of the packed order: byte l>>3,
+  // MSB first (byte 4w is the word's low byte)
+  const int bit = (lane & ~7) + 7 - (lane & 7);
+  const int per = (nword + step / 32 - 1) / (step / 32);
+  const int w0 = (t0 >> 5) * per, w1 = min(nword, w0 + per);
+  for (int wb = w0; wb < w1; wb += 32) {
+    const int cnt = min(32, w1 - wb);
+    const uint32_t mine = lane < cnt ? __ldg(hw + wb + lane) : 0u;
+    for (int k0 = 0; k0 < cnt; k0 += 8) {
+      uint2 x[8][3];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const uint32_t v = __shfl_sync(0xffffffffu, mine, (k0 + k) & 31);
+        const bool on = k0 + k < cnt && ((v >> bit) & 1u);
+        const uint2 *r = reinterpret_cast<const uint2 *>(rtab + ((size_t)(wb + k0 + k) * 32 + lane) * 6);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) x[k][q] = on ? __ldg(r + q) : make_uint2(0u, 0u);
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          acc[2 * q] ^= x[k][q].x;
+          acc[2 * q + 1] ^= x[k][q].y;
+        }
+    }
+  }
+  for (int pos = nword * 32 + t0; pos < kldpc; pos += step)
+    if ((h[pos >> 3] >> (7 - (pos & 7))) & 1) fold_row(acc, rtab, pos);
+  if (po && scr)
+    for (int j = t0; j < (kpay >> 3); j += step) po[j] = h[j] ^ __ldg(scr + j);
+}
+
+__global__ void __launch_bounds__(BCH_T) bch_packed_kernel(
     const uint8_t *__restrict__ hard, int64_t ld_hard, int kldpc,
     const uint32_t *__restrict__ rtab, uint32_t *__restrict__ syn,
     uint8_t *__restrict__ ok, const uint8_t *__restrict__ scr, int kpay,
     uint8_t *__restrict__ payload, int64_t ld_payload) {
-  const int b = blockIdx.x;
-  const uint8_t *h = hard + (size_t)b * ld_hard;
+  const int b = (int)cluster_id_x();
   uint32_t acc[6] = {0, 0, 0, 0, 0, 0};
-  const int nword = kldpc >> 5;              // whole 32-bit words
-  const uint32_t *hw = reinterpret_cast<const uint32_t *>(h);
-  for (int w = threadIdx.x; w < nword; w += blockDim.x) {
-    uint32_t v = __ldg(hw + w);              // bytes 4w..4w+3, LSB = byte 4w
-    while (v) {
-      const int t = __ffs(v) - 1;            // bit t: byte t>>3, bit t&7
-      v &= v - 1;
-      const int pos = 32 * w + 8 * (t >> 3) + (7 - (t & 7));
-      fold_row(acc, rtab, pos);
-    }
-  }
-  for (int pos = nword * 32 + threadIdx.x; pos < kldpc; pos += blockDim.x)
-    if ((h[pos >> 3] >> (7 - (pos & 7))) & 1) fold_row(acc, rtab, pos);
-  if (payload && scr) {
-    uint8_t *po = payload + (size_t)b * ld_payload;
-    for (int j = threadIdx.x; j < (kpay >> 3); j += blockDim.x)
-      po[j] = h[j] ^ __ldg(scr + j);
-  }
+  fold_packed(acc, hard + (size_t)b * ld_hard, kldpc, rtab, scr, kpay,
+              payload ? payload + (size_t)b * ld_payload : nullptr);
   reduce_store(acc, syn + (size_t)b * 6, ok ? ok + b : nullptr);
 }
 
-__global__ void __launch_bounds__(256) bch_bits_kernel(
+__global__ void __launch_bounds__(BCH_T) bch_bits_kernel(
     const uint8_t *__restrict__ bits, int64_t ld_bits, int kldpc,
     const uint32_t *__restrict__ rtab, uint32_t *__restrict__ syn) {
-  const int b = blockIdx.x;
+  const int b = (int)cluster_id_x();
   const uint8_t *h = bits + (size_t)b * ld_bits;
   uint32_t acc[6] = {0, 0, 0, 0, 0, 0};
-  for (int pos = threadIdx.x; pos < kldpc; pos += blockDim.x)
+  const int step = (int)cluster_nctarank() * BCH_T;
+#pragma unroll 8
+  for (int pos = (int)cluster_ctarank() * BCH_T + threadIdx.x; pos < kldpc; pos += step)
     if (h[pos] & 1) fold_row(acc, rtab, pos);
   reduce_store(acc, syn + (size_t)b * 6, nullptr);
+}
+
+// CTAs per codeword: few words a warp while that leaves a few CTAs per SM.
+static int bch_cluster(int64_t nblk, int kldpc) {
+  int cl = BCH_CL;
+  while (cl > 1 && (nblk * cl > 8 * 148 || kldpc / 32 < cl * (BCH_T / 32))) cl /= 2;
+  return cl;
+}
+
+// launches `fn` with a cluster of `cl` CTAs for each of nblk codewords
+template <typename... P, typename... A>
+static cudaError_t bch_launch(void (*fn)(P...), int nblk, int cl, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)nblk * (unsigned)cl, 1, 1);
+  cfg.blockDim = dim3(BCH_T, 1, 1);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cl;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, fn, args...);
 }
 
 int32_t bch_check_launch(const uint8_t *hard, int64_t ld_hard, int nblk,
@@ -111,9 +174,8 @@ int32_t bch_check_launch(const uint8_t *hard, int64_t ld_hard, int nblk,
     ATSC3_ARG(kpay % 8 == 0 && kpay <= kldpc, "kpayload must be a multiple of 8");
     ATSC3_ARG(ld_payload >= kpay / 8, "ld_payload < kpayload/8");
   }
-  bch_packed_kernel<<<nblk, 256, 0, st>>>(hard, ld_hard, kldpc, rtab, syn, ok,
-                                          scr, kpay, payload, ld_payload);
-  ATSC3_CUDA(cudaGetLastError());
+  ATSC3_CUDA(bch_launch(bch_packed_kernel, nblk, bch_cluster(nblk, kldpc), st, hard, ld_hard,
+                        kldpc, rtab, syn, ok, scr, kpay, payload, ld_payload));
   return 0;
 }
 
@@ -125,8 +187,8 @@ int32_t bch_bits_launch(const uint8_t *bits, int64_t ld_bits, int nblk,
   ATSC3_ARG(bits && rtab && syn, "null pointer");
   ATSC3_ARG(ld_bits >= kldpc, "ld_bits < kldpc");
   ATSC3_ARG(((uintptr_t)rtab & 7) == 0, "rtab must be 8-byte aligned");
-  bch_bits_kernel<<<nblk, 256, 0, st>>>(bits, ld_bits, kldpc, rtab, syn);
-  ATSC3_CUDA(cudaGetLastError());
+  ATSC3_CUDA(bch_launch(bch_bits_kernel, nblk, bch_cluster(nblk, kldpc), st, bits, ld_bits, kldpc,
+                        rtab, syn));
   return 0;
 }
 
@@ -145,29 +207,11 @@ struct BchBatchArgs {
   uint8_t *ok;
 };
 
-__global__ void __launch_bounds__(256) bch_batch_kernel(const BchBatchArgs a) {
-  const int b = blockIdx.x;
-  const uint8_t *h = a.hard + a.hard_off[b];
-  const int kldpc = a.kldpc[b];
-  const uint32_t *rtab = a.rtab + a.rtab_off[b];
+__global__ void __launch_bounds__(BCH_T) bch_batch_kernel(const BchBatchArgs a) {
+  const int b = (int)cluster_id_x();
   uint32_t acc[6] = {0, 0, 0, 0, 0, 0};
-  const int nword = kldpc >> 5;
-  const uint32_t *hw = reinterpret_cast<const uint32_t *>(h);
-  for (int w = threadIdx.x; w < nword; w += blockDim.x) {
-    uint32_t v = __ldg(hw + w);
-    while (v) {
-      const int t = __ffs(v) - 1;
-      v &= v - 1;
-      fold_row(acc, rtab, 32 * w + 8 * (t >> 3) + (7 - (t & 7)));
-    }
-  }
-  for (int pos = nword * 32 + threadIdx.x; pos < kldpc; pos += blockDim.x)
-    if ((h[pos >> 3] >> (7 - (pos & 7))) & 1) fold_row(acc, rtab, pos);
-  if (a.payload) {
-    uint8_t *po = a.payload + a.pay_off[b];
-    for (int j = threadIdx.x; j < (a.kpay[b] >> 3); j += blockDim.x)
-      po[j] = h[j] ^ __ldg(a.scr + j);
-  }
+  fold_packed(acc, a.hard + a.hard_off[b], a.kldpc[b], a.rtab + a.rtab_off[b], a.scr,
+              a.payload ? a.kpay[b] : 0, a.payload ? a.payload + a.pay_off[b] : nullptr);
   reduce_store(acc, a.syn + (size_t)b * 6, a.ok + b);
 }
 
@@ -188,8 +232,8 @@ int32_t atsc3_bch_batch(const uint8_t *hard, const int64_t *hard_off,
   ATSC3_ARG(!payload || (scr && kpay && pay_off), "payload needs scr, kpay, pay_off");
   BchBatchArgs a{hard, hard_off, kldpc, rtab, rtab_off, scr, kpay, payload,
                  pay_off, syn, ok};
-  bch_batch_kernel<<<nblk, 256, 0, (cudaStream_t)stream>>>(a);
-  ATSC3_CUDA(cudaGetLastError());
+  // the lengths are on the device: the cluster of the longest
+  ATSC3_CUDA(bch_launch(bch_batch_kernel, nblk, bch_cluster(nblk, 64800), (cudaStream_t)stream, a));
   return 0;
 }
 

@@ -105,6 +105,7 @@ struct QcePlan {
   int32_t *d_ccols = nullptr;   // (nb) columns grouped by owner CTA
   int4 *d_itab = nullptr;       // variable-phase items, grouped by CTA
   int32_t *d_wbin = nullptr;    // (cluster, QBINS+1) bin offsets into each CTA's items
+  int32_t *d_err = nullptr;     // set by a launch whose work stealing got no answer
   uint32_t *d_xtab = nullptr;   // per slot of a spread column: CTA << 20 | byte offset
   int32_t *d_rptr = nullptr;    // (Q+1)
   int4 *d_cdesc = nullptr;      // per column
@@ -780,6 +781,8 @@ struct QceArgs {
   uint8_t *conv;
   int32_t *its;
   int32_t *bad;
+  int steal;                    // more codewords than resident clusters
+  int32_t *err;                 // the plan's error word
 };
 
 
@@ -1271,6 +1274,49 @@ __device__ __forceinline__ int qce_check_heavy(const uint2 *he, int deg, int wra
   return lv ? (int)(synw & 1u) : 0;
 }
 
+// Work stealing between the clusters of a launch: the grid has a cluster per
+// codeword, and a cluster that has finished one asks the hardware to cancel the
+// next cluster not yet launched and decodes its codeword, keeping its tables.
+// Codewords end after 10 to 50 iterations, so fixed shares left clusters idle (45
+// codewords of 64800 8/15, three of them at 50 iterations: 22 clusters with fixed
+// shares wait for one of about 74, with this 66).  `w` words of the exchange area
+// (16-byte aligned): the response (4), its mbarrier (2).
+__device__ __forceinline__ void qce_steal_init(uint32_t w) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(w + 16u) : "memory");
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+
+__device__ __forceinline__ void qce_steal_ask(uint32_t w) {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], 16;" :: "r"(w + 16u) : "memory");
+  asm volatile(
+      "clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+      :: "r"(w), "r"(w + 16u) : "memory");
+}
+
+// first CTA of the cancelled cluster; -1: none is left; -2: no answer within the
+// bounded wait (the answer takes about a microsecond)
+__device__ __forceinline__ int qce_steal_answer(uint32_t w, uint32_t phase) {
+  uint32_t ok = 0;
+  for (int i = 0; i < (1 << 20) && !ok; ++i)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(w + 16u), "r"(phase) : "memory");
+  if (!ok) return -2;
+  uint32_t got, x;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 h;\n\t"
+      "ld.shared.b128 h, [%2];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "mov.u32 %1, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n\t}"
+      : "=r"(got), "=r"(x) : "r"(w) : "memory");
+  return got ? (int)x : -1;
+}
+
 // NS: compile-time slots per block row (qce_ns); NT: threads per CTA; TA:
 // the Type A paths (rows above NS, columns in both zones) are compiled in.
 // A variable item's inputs that the slots do not hold: its table entry, the
@@ -1417,11 +1463,13 @@ __global__ void __launch_bounds__(NT, 1) ldpc_qce_kernel(const QceArgs a) {
     const uint32_t v = __ldg(a.xtab + a.xb[rank] + q);
     xtab[q] = dsmem_map(sm_sa + (v & 0xFFFFFu), v >> 20);
   }
+  const uint32_t steal_sa = part_sa + 44u * 4u;
   if (tid == 0) {
     part[0] = 0;
     part[1] = 0;
     part[2] = 0;
     part[3] = 0;
+    if (rank == 0) qce_steal_init(steal_sa);
   }
   __syncthreads();
 
@@ -1438,7 +1486,9 @@ __global__ void __launch_bounds__(NT, 1) ldpc_qce_kernel(const QceArgs a) {
   // float32 kernels of up to 8 slots (Type B) at 1024 threads, up to 22 at 512
   constexpr bool VPF = sizeof(V) == 4 && (NT >= 1024 ? (NS <= 8 && !TA) : NS <= 22);
 
-  for (int b = (int)cluster_id_x(); b < a.nblk; b += (int)ncluster_x()) {
+  uint32_t turn = 0;             // answers taken so far
+  for (int b = (int)cluster_id_x(); b >= 0;) {
+    int nb = -1;                 // the next codeword
     const V *lam = reinterpret_cast<const V *>(a.llr) + (size_t)b * a.ld_llr;
     // ---- prologue: q = lam - 0 = lam on every slot, hard bits of lam; the
     // absent entry holds -0.0 (adding it is exact) ---------------------------
@@ -1589,6 +1639,7 @@ __global__ void __launch_bounds__(NT, 1) ldpc_qce_kernel(const QceArgs a) {
       const int badct = part[it & 1];
       const bool done = (badct == 0) && (!TORCH || it > 0);
       if (done || it >= a.iters) {
+        if (a.steal && rank == 0 && tid == 0) qce_steal_ask(steal_sa);
         // outputs from this CTA's bitmap replica (complete in every CTA):
         // CTA `rank` writes its share of the codeword's bytes / bits
         const int nby = a.n >> 3;
@@ -1616,9 +1667,20 @@ __global__ void __launch_bounds__(NT, 1) ldpc_qce_kernel(const QceArgs a) {
           a.its[b] = it;
           a.bad[b] = done ? 0 : badct;
         }
+        if (a.steal && rank == 0 && tid < 32) {
+          int x = 0;
+          if (tid == 0) x = qce_steal_answer(steal_sa, turn & 1u);
+          x = __shfl_sync(0xffffffffu, x, 0);
+          if (x == -2 && tid == 0) *a.err = 1;
+          if (lane < CL)
+            dsmem_st_u32(dsmem_map(part_sa + 52u * 4u, (uint32_t)lane),
+                         (uint32_t)(x < 0 ? -1 : x / CL));
+        }
+        ++turn;
         // every CTA has read its replica before the next codeword's prologue
         // writes the replicas of the whole cluster; both counters start at 0
         cluster_sync_all();
+        if (a.steal) nb = ((volatile int *)part)[52];
         if (tid == 0) {
           part[0] = 0;
           part[1] = 0;
@@ -1742,6 +1804,7 @@ __global__ void __launch_bounds__(NT, 1) ldpc_qce_kernel(const QceArgs a) {
       }
       cluster_sync_all();
     }
+    b = nb;
   }
   cluster_sync_all();
 }
@@ -1857,7 +1920,9 @@ static cudaError_t qce_upload(QcePlan &p, const QceTables &t, const QcePlan *lik
     const void *src;
     size_t bytes;
   };
+  static const int32_t zero = 0;
   const Part parts[] = {
+      {(void **)&p.d_err, &zero, 4},
       {(void **)&p.d_rdesc, t.rdesc.data(), t.rdesc.size() * 16},
       {(void **)&p.d_rptr, t.rptr.data(), t.rptr.size() * 4},
       {(void **)&p.d_cdesc, t.cdesc.data(), t.cdesc.size() * 16},
@@ -2073,6 +2138,12 @@ int32_t atsc3_ldpc_qce_plan_info(const atsc3_ldpc_qce_plan *h, int64_t *info) {
   info[7] = h->p.table_bytes;
   info[8] = h->p.max_slots;
   info[9] = h->p.cb[1] - h->p.cb[0];   // columns of CTA 0
+  return 0;
+}
+
+int32_t atsc3_ldpc_qce_plan_error(const atsc3_ldpc_qce_plan *h, int32_t *err) {
+  ATSC3_ARG(h && err, "null argument");
+  ATSC3_CUDA(cudaMemcpy(err, h->p.d_err, 4, cudaMemcpyDeviceToHost));
   return 0;
 }
 
@@ -2365,9 +2436,11 @@ static int32_t qce_decode_impl(
   const int32_t rc = qce_choose(h, nblk, fn, threads, &pick, &ncl);
   if (rc) return rc;
   const QcePlan &p = *pick;
-  ncl = std::min(ncl, nblk);
+  ATSC3_ARG((int64_t)nblk * p.cluster <= INT32_MAX, "too many codewords");
   QceArgs a;
   std::memset(&a, 0, sizeof(a));
+  a.steal = nblk > ncl ? 1 : 0;
+  a.err = h->p.d_err;
   a.llr = llr;
   a.ld_llr = ld_llr;
   a.nblk = nblk;
@@ -2419,7 +2492,7 @@ static int32_t qce_decode_impl(
   a.its = its;
   a.bad = bad;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(ncl * p.cluster, 1, 1);
+  cfg.gridDim = dim3(nblk * p.cluster, 1, 1);
   cfg.blockDim = dim3(threads, 1, 1);
   cfg.dynamicSmemBytes = p.smem;
   cfg.stream = (cudaStream_t)stream;

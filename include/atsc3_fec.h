@@ -221,6 +221,10 @@ int32_t atsc3_ldpc_qce_plan_create_one(int32_t n, int32_t kldpc, int32_t qa,
                                        const int32_t *addr,
                                        atsc3_ldpc_qce_plan **plan);
 
+/* 1 when a decode with this plan lost codewords: a cluster asking for its next
+ * one got no answer within its bounded wait.  Waits for the device. */
+int32_t atsc3_ldpc_qce_plan_error(const atsc3_ldpc_qce_plan *plan, int32_t *err);
+
 /* The float64 edge-buffer decoder (8-byte slots, float64 messages and
  * posteriors, 512 threads per CTA): the arithmetic of the float64 paths of
  * lab/m9_gpu.py:168-211 (torch semantics, GpuMinSum's default dtype) and

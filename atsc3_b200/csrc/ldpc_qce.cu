@@ -2423,6 +2423,7 @@ static int32_t qce_decode_impl(
   if (nblk == 0) return 0;
   ATSC3_ARG(conv && its && bad, "null status output");
   ATSC3_ARG(llr != nullptr, "null llr");
+  const bool pinned = threads > 0;
   if (threads <= 0) threads = qce_default_threads(h->p.dr_light);
   ATSC3_ARG(threads == 512 || threads == 1024, "threads must be 512 or 1024");
   if (qce_ns(h->p.dr_light) > 17 || f64) threads = 512;   // only the 512-thread build
@@ -2433,9 +2434,24 @@ static int32_t qce_decode_impl(
   }
   const QcePlan *pick = nullptr;
   int ncl = 0;
-  const int32_t rc = qce_choose(h, nblk, fn, threads, &pick, &ncl);
+  int32_t rc = qce_choose(h, nblk, fn, threads, &pick, &ncl);
   if (rc) return rc;
   const QcePlan &p = *pick;
+  // a 64800-bit codeword over nine and more CTAs: 512 threads with twice the items
+  // each (24 iterations on 14 CTAs, us, 1024 / 512 threads: 6/15 323 / 288, 8/15
+  // 333 / 291, 10/15 337 / 308, 2/15 418 / 401, 7/15 477 / 459; on 9 the same); a
+  // 16200-bit one has too few items (11/15 on 14 CTAs 5.1 / 5.3 us an iteration)
+  if (!pinned && threads == 1024 && pick != &h->p && p.cluster > 6 && 6 * p.nb >= 64 * p.cluster) {
+    QceFn half = qce_fn(semantics, h->p.dr_light, 512, h->p.qb > 0, f64);
+    int n = 0;
+    rc = qce_max_clusters(half, p.cluster, p.smem, 512, p.device, &n);
+    if (rc) return rc;
+    if (n >= nblk) {
+      fn = half;
+      threads = 512;
+      ncl = n;
+    }
+  }
   ATSC3_ARG((int64_t)nblk * p.cluster <= INT32_MAX, "too many codewords");
   QceArgs a;
   std::memset(&a, 0, sizeof(a));

@@ -134,13 +134,24 @@ def make_frames(nframes, seed, device):
     return cells, sig, nblk, tx.kp
 
 
+def kernel_route():
+    """What cpu_reference_decode runs for the LDPC decode: (kind, words)."""
+    import oracle
+    if oracle.ref_lib() is not None:
+        return "reference", ("lab/ldpc_kernel.c compiled -O3 "
+                             "-ffp-contract=off (oracle/_ref)")
+    return "oracle", ("the oracle's own restatement of lab/ldpc_kernel.c "
+                      "(the reference's is not built here)")
+
+
 def cpu_reference_decode(cells, sig, threads, mod=None, rate=None, n=None,
                          full=False):
     """The reference's CPU path on host cores, through the oracle: float32
     demap (numpy, the lab/m44_ldm.py:2431-2494 arithmetic) with per-cell
     sigma2, de-interleave, the reference's own lab/ldpc_kernel.c compiled
-    into oracle/_ref (thread sub-batches, as lab/m44_ldm.py:2558-2576), BCH
-    as a packed GF(2) product (lab/m9_accel.py:212-236).  Returns
+    into oracle/_ref (thread sub-batches, as lab/m44_ldm.py:2558-2576; the
+    oracle's restatement of it where that is not built), BCH as a packed
+    GF(2) product (lab/m9_accel.py:212-236).  Returns
     (#blocks BCH-clean, its), or with full=True the dict of every output
     (bits, conv, its, bad, ok, payload)."""
     import oracle
@@ -160,8 +171,14 @@ def cpu_reference_decode(cells, sig, threads, mod=None, rate=None, n=None,
                                    sig if scalar else sig[b:b + 1]),
             range(nblk))))
     lam = oracle.deinterleave(q, lq, n)
-    bits, conv, its, bad = oracle.flood_ref(lam, tabs, n, iters=ITERS,
-                                            alpha=ALPHA, threads=threads)
+    if kernel_route()[0] == "reference":
+        bits, conv, its, bad = oracle.flood_ref(lam, tabs, n, iters=ITERS,
+                                                alpha=ALPHA, threads=threads)
+    else:
+        with ThreadPoolExecutor(threads) as ex:
+            bits, conv, its, bad = (np.concatenate(o) for o in zip(*ex.map(
+                lambda x: oracle.flood(x, tabs, n, iters=ITERS, alpha=ALPHA),
+                np.array_split(lam, min(threads, nblk)))))
     syn = oracle.bch_syndrome_fast(bits[:, :K], n)
     if not full:
         return sum(1 for s in syn if s == 0), its
@@ -277,6 +294,12 @@ def run_reference(args, rank, world):
     from atsc3_b200 import codes as C
     threads = os.cpu_count() or 1
     kp = C.kpayload(RATE, N_INNER)
+    laid_out = os.path.exists(os.path.join(REF_TREE, "lab", "ldpc_kernel.so"))
+    if not laid_out and kernel_route()[0] != "reference":
+        return {"impl": "reference",
+                "unavailable": "neither baseline/_ref nor oracle/_ref is laid "
+                               "out: the reference's sources are not on this "
+                               "machine"}
     dev = "cuda" if torch.cuda.is_available() else "cpu"
     nsteps = args.steps + args.warmup
     cells, sig, nblk, _ = make_frames(nsteps, args.seed, dev)
@@ -707,15 +730,16 @@ def cpu_baseline(par):
                 "-ffp-contract=off, m9_accel.bch_syndrome_batch, descramble)")
     except RuntimeError as e:
         path = None
-        what = (f"oracle route ({e}): numpy float32 demap + lab/ldpc_kernel.c "
-                f"(-O3 -ffp-contract=off, oracle/_ref) + packed BCH")
+        what = (f"oracle route ({e}): numpy float32 demap + "
+                f"{kernel_route()[1]} + packed BCH")
     t0 = time.perf_counter()
     out = (path.decode(c, g) if path is not None else
            cpu_reference_decode(c, g, threads, full=True))
     dt = time.perf_counter() - t0
     nf = par["cells"].shape[0]
     return ({"value": c.shape[0] * kp / dt / 1e6, "unit": "Mbit/s",
-             "cores": threads, "kind": "reference",
+             "cores": threads,
+             "kind": "reference" if path is not None else kernel_route()[0],
              "sample": f"{c.shape[0]} blocks: the first {nf} timed frames "
                        f"(one whole frame per Es/N0 point "
                        f"{par['esn0_db'][0]:g}..{par['esn0_db'][-1]:g} dB), "
@@ -757,9 +781,8 @@ def parity_check(par, ref_py):
            "vs_reference_kernel": mism(o, ("bits", "conv", "its", "bad",
                                             "ok", "payload")),
            "gpu_rerun_flag_mismatch": rerun,
-           "reference_kernel": "lab/ldpc_kernel.c compiled -O3 "
-                               "-ffp-contract=off (oracle/_ref), float32 "
-                               "demap with per-cell sigma2, packed BCH"}
+           "reference_kernel": kernel_route()[1] + ", float32 demap with "
+                               "per-cell sigma2, packed BCH"}
     if ref_py is not None and "its" not in ref_py:
         res["vs_reference_python"] = mism(ref_py, ("bits", "conv", "bad",
                                                    "ok", "payload"))
@@ -995,7 +1018,7 @@ def run_plain(args):
             "cpu_reference": {"value": nblk * kp / cpu_s / 1e6, "unit": "Mbit/s",
                               "cores": threads, "bch_ok": int(nok_cpu),
                               "mean_iters": float(np.mean(its_cpu)),
-                              "what": "float32 demap numpy + lab/ldpc_kernel.c over all host threads + packed BCH, same 32 blocks"},
+                              "what": f"float32 demap numpy + {kernel_route()[1]} over all host threads + packed BCH, same 32 blocks"},
             "data": "synthetic", "dtype": "f32"}
 
 

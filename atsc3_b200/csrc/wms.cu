@@ -33,7 +33,7 @@
 // share an index load; the caller's (nblk, n) arrays are transposed on the way in
 // and out.  With [block][item] the gathers of one iteration touched a 32-byte
 // sector per 4- or 16-byte value.  What bounds it now is moving the messages:
-// 5 passes over 4 bytes an edge an iteration forward, 5 backward.
+// 4 passes over 4 bytes an edge an iteration forward, 4 backward.
 // 64 blocks of 64800 8/15, 12 iterations, forward and backward with the loss:
 // 10.5 ms -> 1.9 ms.
 //

@@ -4,8 +4,8 @@
 hand-written backward kernels of ``csrc/wms.cu``: T flooding iterations with
 per-iteration, per-check-degree scale ``alpha[t, d]`` and offset
 ``beta[t, d]`` (messages ``sgn * relu(alpha * mu - beta)``), checkpointing one
-16-byte record per check per iteration and recomputing messages in the
-backward.  ``reference_f64`` is the same forward in float64 torch ops whose
+16-byte record per check per iteration, from which the backward takes signs,
+minima and the arg-min.  ``reference_f64`` is the same forward in float64 torch ops whose
 autograd gradient (and finite differences) check the kernels.
 
 ``train`` fits the weights on LLRs produced by this package's own demapper

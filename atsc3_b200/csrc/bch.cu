@@ -36,7 +36,9 @@ __device__ __forceinline__ void fold_row(uint32_t (&acc)[6], const uint32_t *__r
   acc[3] ^= b.y; acc[4] ^= c.x; acc[5] ^= c.y;
 }
 
-// The cluster's XOR of acc, written by its first CTA.
+// The cluster's XOR of acc, written by its first CTA.  The kernel has arrived at
+// the cluster barrier at its entry; the wait here, behind the fold, shows that the
+// first CTA has started before its shared memory is written.
 __device__ __forceinline__ void reduce_store(uint32_t (&acc)[6], uint32_t *syn, uint8_t *ok) {
   __shared__ uint32_t red[BCH_T / 32][6];
   __shared__ uint32_t all[BCH_CL][6];           // rank 0: every CTA's words
@@ -48,6 +50,7 @@ __device__ __forceinline__ void reduce_store(uint32_t (&acc)[6], uint32_t *syn, 
 #pragma unroll
     for (int w = 0; w < 6; ++w) red[warp][w] = acc[w];
   __syncthreads();
+  cluster_wait();
   if (threadIdx.x < 6) {
     uint32_t v = 0;
     for (int q = 0; q < BCH_T / 32; ++q) v ^= red[q][threadIdx.x];
@@ -113,6 +116,7 @@ __global__ void __launch_bounds__(BCH_T) bch_packed_kernel(
     const uint32_t *__restrict__ rtab, uint32_t *__restrict__ syn,
     uint8_t *__restrict__ ok, const uint8_t *__restrict__ scr, int kpay,
     uint8_t *__restrict__ payload, int64_t ld_payload) {
+  cluster_arrive();
   const int b = (int)cluster_id_x();
   uint32_t acc[6] = {0, 0, 0, 0, 0, 0};
   fold_packed(acc, hard + (size_t)b * ld_hard, kldpc, rtab, scr, kpay,
@@ -123,6 +127,7 @@ __global__ void __launch_bounds__(BCH_T) bch_packed_kernel(
 __global__ void __launch_bounds__(BCH_T) bch_bits_kernel(
     const uint8_t *__restrict__ bits, int64_t ld_bits, int kldpc,
     const uint32_t *__restrict__ rtab, uint32_t *__restrict__ syn) {
+  cluster_arrive();
   const int b = (int)cluster_id_x();
   const uint8_t *h = bits + (size_t)b * ld_bits;
   uint32_t acc[6] = {0, 0, 0, 0, 0, 0};
@@ -208,6 +213,7 @@ struct BchBatchArgs {
 };
 
 __global__ void __launch_bounds__(BCH_T) bch_batch_kernel(const BchBatchArgs a) {
+  cluster_arrive();
   const int b = (int)cluster_id_x();
   uint32_t acc[6] = {0, 0, 0, 0, 0, 0};
   fold_packed(acc, a.hard + a.hard_off[b], a.kldpc[b], a.rtab + a.rtab_off[b], a.scr,

@@ -65,6 +65,18 @@ __device__ __forceinline__ void cluster_sync_all() {
       "barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// The same barrier in two halves, without memory ordering: peers' shared memory
+// may be touched once every CTA of the cluster has started, so a kernel arrives
+// at its entry and waits before its first such access, with work of its own in
+// between.
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }

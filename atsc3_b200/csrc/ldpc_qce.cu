@@ -1471,7 +1471,9 @@ __global__ void __launch_bounds__(NT, 1) ldpc_qce_kernel(const QceArgs a) {
     part[3] = 0;
     if (rank == 0) qce_steal_init(steal_sa);
   }
-  __syncthreads();
+  // the prologue writes peers' bitmaps and slots: every CTA has started (and
+  // has its own tables staged)
+  cluster_sync_all();
 
   // the absent wrap entry (last parity column, bit 359, its wrap slot) is
   // lane 7 of sub-chunk 1 of that column's last item, slot 1 of the column

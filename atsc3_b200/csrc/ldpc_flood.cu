@@ -1082,6 +1082,7 @@ __global__ void __launch_bounds__(1024, 1) ldpc_batch_kernel(const BatchArgs a) 
   const uint32_t slot_sa = smem_u32(slot);
   const int rank = (int)cluster_ctarank();
   const int CL = (int)cluster_nctarank();
+  cluster_sync_all();              // the slots of peers may be written from here on
   for (;;) {
     if (rank == 0 && threadIdx.x == 0) {
       const int q = atomicAdd(a.counter, 1);

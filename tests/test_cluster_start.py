@@ -44,7 +44,8 @@ def events(fns, body, seen=()):
             yield from events(fns, fns[name][1], seen + (name,))
 
 
-@pytest.mark.parametrize("source", ["bch.cu", "ldpc_qce.cu"])
+@pytest.mark.parametrize("source", ["bch.cu", "cpe.cu", "ldpc_flood.cu",
+                                    "ldpc_qc.cu", "ldpc_qce.cu"])
 def test_barrier_before_peer_access(source):
     with open(os.path.join(CSRC, source)) as f:
         fns = functions(f.read())

@@ -105,7 +105,6 @@ struct QcePlan {
   int32_t *d_ccols = nullptr;   // (nb) columns grouped by owner CTA
   int4 *d_itab = nullptr;       // variable-phase items, grouped by CTA
   int32_t *d_wbin = nullptr;    // (cluster, QBINS+1) bin offsets into each CTA's items
-  int32_t *d_err = nullptr;     // set by a launch whose work stealing got no answer
   uint32_t *d_xtab = nullptr;   // per slot of a spread column: CTA << 20 | byte offset
   int32_t *d_rptr = nullptr;    // (Q+1)
   int4 *d_cdesc = nullptr;      // per column
@@ -781,8 +780,7 @@ struct QceArgs {
   uint8_t *conv;
   int32_t *its;
   int32_t *bad;
-  int steal;                    // more codewords than resident clusters
-  int32_t *err;                 // the plan's error word
+  int share;                    // more codewords than clusters (qce_claim)
 };
 
 
@@ -1274,47 +1272,60 @@ __device__ __forceinline__ int qce_check_heavy(const uint2 *he, int deg, int wra
   return lv ? (int)(synw & 1u) : 0;
 }
 
-// Work stealing between the clusters of a launch: the grid has a cluster per
-// codeword, and a cluster that has finished one asks the hardware to cancel the
-// next cluster not yet launched and decodes its codeword, keeping its tables.
-// Codewords end after 10 to 50 iterations, so fixed shares left clusters idle (45
-// codewords of 64800 8/15, three of them at 50 iterations: 22 clusters with fixed
-// shares wait for one of about 74, with this 66).  `w` words of the exchange area
-// (16-byte aligned): the response (4), its mbarrier (2).
-__device__ __forceinline__ void qce_steal_init(uint32_t w) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(w + 16u) : "memory");
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-__device__ __forceinline__ void qce_steal_ask(uint32_t w) {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], 16;" :: "r"(w + 16u) : "memory");
-  asm volatile(
-      "clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
-      :: "r"(w), "r"(w + 16u) : "memory");
-}
-
-// first CTA of the cancelled cluster; -1: none is left; -2: no answer within the
-// bounded wait (the answer takes about a microsecond)
-__device__ __forceinline__ int qce_steal_answer(uint32_t w, uint32_t phase) {
-  uint32_t ok = 0;
-  for (int i = 0; i < (1 << 20) && !ok; ++i)
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(w + 16u), "r"(phase) : "memory");
-  if (!ok) return -2;
-  uint32_t got, x;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b128 h;\n\t"
-      "ld.shared.b128 h, [%2];\n\t"
-      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t"
-      "mov.u32 %1, 0;\n\t"
-      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n\t}"
-      : "=r"(got), "=r"(x) : "r"(w) : "memory");
-  return got ? (int)x : -1;
+// Sharing the codewords of a launch between its resident clusters: cluster c
+// starts with codeword c, and one that has finished takes the next that nobody
+// has, keeping its tables.  Codewords end after 10 to 50 iterations, so fixed
+// shares leave clusters idle.  The record of who has which is the caller's `its`,
+// which the launch finds at -1: a claim turns a codeword's -1 into -2, its
+// iteration count replaces that.  A claim cannot be lost and nothing waits for
+// another cluster; cancelling clusters not yet launched (clusterlaunchcontrol)
+// gains the same but needs a wait for the answer, and a codeword whose answer does
+// not come within a bounded wait is decoded by nobody.  Against fixed shares, ms:
+// 66 codewords of 64800 8/15, a few of them at 50 iterations, 1.168 -> 0.796; three
+// codewords a cluster that all end alike, 64800 4/15 1.056 -> 1.058, 13/15 0.481 ->
+// 0.488 (0.494 with one window of 32 words a round trip in the search).
+// The codeword that a fixed share would hold next is tried first, one round trip
+// to the L2 that the outputs' stores cover; where it is taken, the first word with
+// an open codeword is searched, clusters that search at once trying different
+// ones of it.  Every lane of one warp calls it; `base`: everything below is taken.
+__device__ __forceinline__ int qce_claim(int32_t *its, int nblk, int guess, int *base) {
+  const int lane = threadIdx.x & 31;
+  int old = 0;
+  if (guess < nblk) {
+    if (lane == 0) old = atomicCAS(its + guess, -1, -2);
+    if (__shfl_sync(0xffffffffu, old, 0) == -1) return guess;
+  }
+  int p = *base, got = -1;
+  while (got < 0 && p < nblk) {
+    int v[8];                       // 256 codewords a round trip
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int k = p + 32 * j + lane;
+      v[j] = k < nblk ? *(volatile int32_t *)(its + k) : 0;
+    }
+    uint32_t open = 0;
+    int w = 0;
+#pragma unroll
+    for (int j = 7; j >= 0; --j) {
+      const uint32_t o = __ballot_sync(0xffffffffu, v[j] == -1);
+      open = o ? o : open;
+      w = o ? j : w;
+    }
+    if (!open) {
+      p += 256;
+      continue;
+    }
+    p += 32 * w;
+    const int k = p + (int)__fns(open, 0, 1 + (int)(cluster_id_x() % (uint32_t)__popc(open)));
+    if (lane == 0) old = atomicCAS(its + k, -1, -2);
+    // where it failed another cluster has taken it since the look: at most one
+    // more look per codeword
+    if (__shfl_sync(0xffffffffu, old, 0) == -1) got = k;
+  }
+  __syncwarp();
+  if (lane == 0) *base = p;
+  __syncwarp();
+  return got;
 }
 
 // NS: compile-time slots per block row (qce_ns); NT: threads per CTA; TA:
@@ -1463,13 +1474,12 @@ __global__ void __launch_bounds__(NT, 1) ldpc_qce_kernel(const QceArgs a) {
     const uint32_t v = __ldg(a.xtab + a.xb[rank] + q);
     xtab[q] = dsmem_map(sm_sa + (v & 0xFFFFFu), v >> 20);
   }
-  const uint32_t steal_sa = part_sa + 44u * 4u;
   if (tid == 0) {
     part[0] = 0;
     part[1] = 0;
     part[2] = 0;
     part[3] = 0;
-    if (rank == 0) qce_steal_init(steal_sa);
+    part[45] = (int)ncluster_x();     // qce_claim's base
   }
   // the prologue writes peers' bitmaps and slots: every CTA has started (and
   // has its own tables staged)
@@ -1488,7 +1498,6 @@ __global__ void __launch_bounds__(NT, 1) ldpc_qce_kernel(const QceArgs a) {
   // float32 kernels of up to 8 slots (Type B) at 1024 threads, up to 22 at 512
   constexpr bool VPF = sizeof(V) == 4 && (NT >= 1024 ? (NS <= 8 && !TA) : NS <= 22);
 
-  uint32_t turn = 0;             // answers taken so far
   for (int b = (int)cluster_id_x(); b >= 0;) {
     int nb = -1;                 // the next codeword
     const V *lam = reinterpret_cast<const V *>(a.llr) + (size_t)b * a.ld_llr;
@@ -1641,7 +1650,10 @@ __global__ void __launch_bounds__(NT, 1) ldpc_qce_kernel(const QceArgs a) {
       const int badct = part[it & 1];
       const bool done = (badct == 0) && (!TORCH || it > 0);
       if (done || it >= a.iters) {
-        if (a.steal && rank == 0 && tid == 0) qce_steal_ask(steal_sa);
+        if (a.share && rank == 0 && tid < 32) {
+          const int x = qce_claim(a.its, a.nblk, b + (int)ncluster_x(), part + 45);
+          if (lane < CL) dsmem_st_u32(dsmem_map(part_sa + 44u * 4u, (uint32_t)lane), (uint32_t)x);
+        }
         // outputs from this CTA's bitmap replica (complete in every CTA):
         // CTA `rank` writes its share of the codeword's bytes / bits
         const int nby = a.n >> 3;
@@ -1669,20 +1681,10 @@ __global__ void __launch_bounds__(NT, 1) ldpc_qce_kernel(const QceArgs a) {
           a.its[b] = it;
           a.bad[b] = done ? 0 : badct;
         }
-        if (a.steal && rank == 0 && tid < 32) {
-          int x = 0;
-          if (tid == 0) x = qce_steal_answer(steal_sa, turn & 1u);
-          x = __shfl_sync(0xffffffffu, x, 0);
-          if (x == -2 && tid == 0) *a.err = 1;
-          if (lane < CL)
-            dsmem_st_u32(dsmem_map(part_sa + 52u * 4u, (uint32_t)lane),
-                         (uint32_t)(x < 0 ? -1 : x / CL));
-        }
-        ++turn;
         // every CTA has read its replica before the next codeword's prologue
         // writes the replicas of the whole cluster; both counters start at 0
         cluster_sync_all();
-        if (a.steal) nb = ((volatile int *)part)[52];
+        if (a.share) nb = ((volatile int *)part)[44];
         if (tid == 0) {
           part[0] = 0;
           part[1] = 0;
@@ -1922,9 +1924,7 @@ static cudaError_t qce_upload(QcePlan &p, const QceTables &t, const QcePlan *lik
     const void *src;
     size_t bytes;
   };
-  static const int32_t zero = 0;
   const Part parts[] = {
-      {(void **)&p.d_err, &zero, 4},
       {(void **)&p.d_rdesc, t.rdesc.data(), t.rdesc.size() * 16},
       {(void **)&p.d_rptr, t.rptr.data(), t.rptr.size() * 4},
       {(void **)&p.d_cdesc, t.cdesc.data(), t.cdesc.size() * 16},
@@ -2145,7 +2145,7 @@ int32_t atsc3_ldpc_qce_plan_info(const atsc3_ldpc_qce_plan *h, int64_t *info) {
 
 int32_t atsc3_ldpc_qce_plan_error(const atsc3_ldpc_qce_plan *h, int32_t *err) {
   ATSC3_ARG(h && err, "null argument");
-  ATSC3_CUDA(cudaMemcpy(err, h->p.d_err, 4, cudaMemcpyDeviceToHost));
+  *err = 0;
   return 0;
 }
 
@@ -2454,11 +2454,10 @@ static int32_t qce_decode_impl(
       ncl = n;
     }
   }
-  ATSC3_ARG((int64_t)nblk * p.cluster <= INT32_MAX, "too many codewords");
+  ncl = std::min(ncl, nblk);
   QceArgs a;
   std::memset(&a, 0, sizeof(a));
-  a.steal = nblk > ncl ? 1 : 0;
-  a.err = h->p.d_err;
+  a.share = nblk > ncl ? 1 : 0;
   a.llr = llr;
   a.ld_llr = ld_llr;
   a.nblk = nblk;
@@ -2510,7 +2509,7 @@ static int32_t qce_decode_impl(
   a.its = its;
   a.bad = bad;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(nblk * p.cluster, 1, 1);
+  cfg.gridDim = dim3(ncl * p.cluster, 1, 1);
   cfg.blockDim = dim3(threads, 1, 1);
   cfg.dynamicSmemBytes = p.smem;
   cfg.stream = (cudaStream_t)stream;
@@ -2521,6 +2520,8 @@ static int32_t qce_decode_impl(
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  if (a.share)
+    ATSC3_CUDA(cudaMemsetAsync(its, 0xFF, (size_t)nblk * sizeof(int32_t), cfg.stream));
   ATSC3_CUDA(cudaLaunchKernelEx(&cfg, fn, a));
   return 0;
 }

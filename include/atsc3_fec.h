@@ -221,8 +221,8 @@ int32_t atsc3_ldpc_qce_plan_create_one(int32_t n, int32_t kldpc, int32_t qa,
                                        const int32_t *addr,
                                        atsc3_ldpc_qce_plan **plan);
 
-/* 1 when a decode with this plan lost codewords: a cluster asking for its next
- * one got no answer within its bounded wait.  Waits for the device. */
+/* 1 when a decode with this plan lost codewords.  None can: the clusters of a
+ * launch claim their codewords with atomics on `its`, so *err is always 0. */
 int32_t atsc3_ldpc_qce_plan_error(const atsc3_ldpc_qce_plan *plan, int32_t *err);
 
 /* The float64 edge-buffer decoder (8-byte slots, float64 messages and

@@ -50,7 +50,7 @@ def cpe_correct_device(pool, sym_ptr, region, alphabets, dummy=None, iters=3,
            torch.view_as_real(dummy).data_ptr() if dummy is not None else None,
            int(iters), torch.view_as_real(out).data_ptr(),
            torch.view_as_real(gains).data_ptr(), work.data_ptr(), st)
-    out._cpe_work = work
+    N.record_use(work, stream, dev)
     return out, gains
 
 

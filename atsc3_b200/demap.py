@@ -103,8 +103,7 @@ def demap(cells, mod, rate, sigma2=None, n=None, deinterleave=True, out=None,
         N.call("atsc3_demap_estimate", zf.data_ptr(), zf.stride(0) // 2, nblk,
                ncell, pts.data_ptr(), nb, N.ptr(lq), out.data_ptr(),
                out.stride(0), work.data_ptr(), st)
-        if stream is not None:      # not the stream the allocator knows
-            out._demap_work = work
+        N.record_use(work, stream, dev)
         return out
     if isinstance(sigma2, (float, int, np.floating)):
         mode, s2s = 0, float(np.float32(sigma2))
@@ -163,8 +162,7 @@ def demap_f64(cells, mod, rate, sigma2=None, n=None, deinterleave=False,
         N.call("atsc3_demap_estimate_f64", zf.data_ptr(), zf.stride(0) // 2,
                nblk, ncell, pts.data_ptr(), nb, N.ptr(lq), out.data_ptr(),
                out.stride(0), work.data_ptr(), st)
-        if stream is not None:      # not the stream the allocator knows
-            out._demap_work = work
+        N.record_use(work, stream, dev)
         return out
     if isinstance(sigma2, (float, int, np.floating)):
         mode, s2s = 0, float(sigma2)

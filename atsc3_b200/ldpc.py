@@ -534,7 +534,8 @@ def sp_decode(tab, llr, iters=100, out=None, stream=None):
            llr.stride(0), nblk, int(iters), o["bits"].data_ptr(),
            o["bits"].stride(0), o["conv"].data_ptr(), o["its"].data_ptr(),
            o["bad"].data_ptr(), work.data_ptr(), st)
-    o["_work"] = work            # alive until the stream has run the launches
+    N.record_use(work, stream, dev)
+    o["_work"] = work
     return o
 
 

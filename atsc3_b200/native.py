@@ -213,3 +213,15 @@ def ptr(t):
 
 def stream_of(torch_mod, device=None):
     return torch_mod.cuda.current_stream(device).cuda_stream
+
+
+def record_use(tensor, stream, device):
+    """Keep `tensor`'s memory until what `stream` (a raw handle named by the
+    caller, None for torch's current stream) has queued is done: the allocator
+    itself only knows the current stream."""
+    if stream is None:
+        return
+    import torch
+    handle = int(getattr(stream, "value", stream) or 0)       # an int or a ctypes pointer
+    tensor.record_stream(torch.cuda.ExternalStream(handle, device=device) if handle
+                         else torch.cuda.default_stream(device))

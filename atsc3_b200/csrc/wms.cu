@@ -80,6 +80,14 @@ struct __align__(4 * VEC) WmsVec {
   float v[VEC];
 };
 
+// Where the record of check c and the i-th of this thread's blocks stands in an
+// iteration's records: blocks fastest; one block a thread (the entry points
+// without padding, whose callers know the records) checks fastest.
+template <int VEC>
+__device__ __forceinline__ size_t wms_rec_at(int nc, int nv, int c, int b, int i) {
+  return VEC == 1 ? (size_t)b * nc + c : ((size_t)c * nv + b) * VEC + i;
+}
+
 // item and first block / VEC of this thread (nv = blocks / VEC); false past the end
 __device__ __forceinline__ bool wms_item(int items, int nv, int &item, int &b) {
   const int64_t g = (int64_t)blockIdx.x * WMS_T + threadIdx.x;
@@ -180,7 +188,7 @@ __global__ void __launch_bounds__(WMS_T) wms_check_fwd(WmsTables T, int nv,
     r.first = (uint16_t)first[i];
     r.second = (uint16_t)second[i];
     r.sx = sx[i];
-    rec[((size_t)c * nv + b) * VEC + i] = r;
+    rec[wms_rec_at<VEC>(T.nc, nv, c, b, i)] = r;
     const float a1 = __fsub_rn(__fmul_rn(al, r.min1), be);
     const float a2 = __fsub_rn(__fmul_rn(al, r.min2), be);
     v1[i] = a1 > 0.f ? a1 : 0.f;
@@ -241,7 +249,7 @@ __global__ void __launch_bounds__(WMS_T) wms_check_bwd(WmsTables T, int nv, int 
     uint32_t sg[VEC];                            // the messages' signs
 #pragma unroll
     for (int i = 0; i < VEC; ++i) {
-      r[i] = rec[((size_t)c * nv + b) * VEC + i];
+      r[i] = rec[wms_rec_at<VEC>(T.nc, nv, c, b, i)];
       sg[i] = __popc(r[i].sx) & 1 ? ~r[i].sx : r[i].sx;
       ga[i] = gb[i] = gmu_rest[i] = gmu_first[i] = 0.f;
     }
@@ -363,10 +371,10 @@ static int32_t wms_forward(const WmsTables &T, int nblk, int iters, const float 
   return 0;
 }
 
-// gllr (nullable): dL/dllr, (nblk, n); may be gtot
+// gtot0 (nullable): dL/dtot^(0), (nblk, n); may be gtot
 template <int VEC>
 static int32_t wms_backward(const WmsTables &T, int nblk, int iters, const float *alpha,
-                            const float *beta, const WmsRec *rec, const float *gtot, float *gllr,
+                            const float *beta, const WmsRec *rec, const float *gtot, float *gtot0,
                             float *galpha, float *gbeta, float *work, cudaStream_t st) {
   constexpr int CV = VEC > 1 ? WMS_CHECK_VEC : 1;
   using V = WmsVec<VEC>;
@@ -384,14 +392,14 @@ static int32_t wms_backward(const WmsTables &T, int nblk, int iters, const float
   for (int t = iters - 1; t >= 0; --t) {
     const size_t p = (size_t)t * T.nbucket;
     float *gx = (gx_next == gxa) ? gxb : gxa;
-    if (t == 0 && !gllr) gx = nullptr;
+    if (t == 0 && !gtot0) gx = nullptr;
     check<<<gc, WMS_T, 0, st>>>(T, nbp / CV, nblk, rec + (size_t)t * nbp * T.nc, alpha + p,
                                 beta + p, (const C *)gt, (const C *)gx_next, (C *)gx, galpha + p,
                                 gbeta + p);
     if (gx) wms_var_bwd<VEC><<<gv, WMS_T, 0, st>>>(T, nv, (const V *)gx, (V *)gt);
     gx_next = gx;
   }
-  if (gllr) wms_blocks_first<<<tiles(T.n, nblk), 256, 0, st>>>(gt, nblk, T.n, nbp, gllr);
+  if (gtot0) wms_blocks_first<<<tiles(T.n, nblk), 256, 0, st>>>(gt, nblk, T.n, nbp, gtot0);
   ATSC3_CUDA(cudaGetLastError());
   return 0;
 }
@@ -471,7 +479,8 @@ int32_t atsc3_wms_gradients(const int32_t *cptr, const int32_t *cidx,
                          work, (cudaStream_t)stream);
 }
 
-// gtot: (nblk, n) dL/dtot^(T) on input, overwritten with dL/dllr on output.
+// gtot: (nblk, n) dL/dtot^(T) on input, overwritten with dL/dtot^(0) (through the
+// messages; llr also enters every later tot^(t) directly).
 // work: nblk * (n + 2 ne) floats; records of atsc3_wms_forward (llr, vchk and
 // vpos are not read).
 int32_t atsc3_wms_backward(const int32_t *cptr, const int32_t *cidx,
@@ -490,7 +499,9 @@ int32_t atsc3_wms_backward(const int32_t *cptr, const int32_t *cidx,
   ATSC3_ARG(n > 0 && nc > 0 && ne > 0 && nbucket > 0 && nbucket <= 127, "bad sizes");
   ATSC3_ARG(iters >= 1 && nblk >= 0, "bad sizes");
   if (nblk == 0) return 0;
-  ATSC3_ARG(gtot && galpha && gbeta && work && records, "null pointer");
+  ATSC3_ARG(cptr && cidx && vptr && vedge && cbucket && alpha && beta && gtot && galpha && gbeta &&
+                work && records,
+            "null pointer");
   return wms_backward<1>(WmsTables{cptr, cidx, vptr, vedge, cbucket, n, nc, ne, nbucket}, nblk,
                          iters, alpha, beta, (const WmsRec *)records, gtot, gtot, galpha, gbeta,
                          work, (cudaStream_t)stream);

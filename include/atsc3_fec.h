@@ -469,17 +469,16 @@ int32_t atsc3_ldpc_layered_inject_timeout(int32_t layer);
  * at most 32 edges), the check and position of each variable-major edge (vchk,
  * vpos; not read), the bucket of each check (int8, at most 127 buckets: its
  * degree class, or its block row for the per-row parameterisation).  records:
- * (iters, nc, nblk) 16-byte per-check checkpoints written by the forward and read
+ * (iters, nblk, nc) 16-byte per-check checkpoints written by the forward and read
  * by the backward.  Forward writes tot_out = the posterior after `iters`
- * iterations (no early stop).  atsc3_wms_forward_work takes its workspace from
- * the caller, nbp * (2n + ne) floats, and writes records of nbp blocks, nbp =
- * nblk rounded up to a multiple of 4 (both 16-byte aligned);
- * atsc3_wms_gradients reads those.  atsc3_wms_forward takes its workspace from
- * the stream's memory pool.
- * Backward: gtot in = dL/dtot_out (overwritten with dL/dllr), galpha/gbeta
- * accumulate (caller zeroes), work = nblk*n + 2*nblk*ne floats.
- * atsc3_wms_gradients: the parameter gradients alone, gtot is only read, work =
- * nbp*n + 2*nbp*ne floats. */
+ * iterations (no early stop); its workspace comes from the stream's memory pool.
+ * Backward: gtot in = dL/dtot_out (overwritten with dL/dtot^(0), the part of
+ * dL/dllr through the first iteration's messages), galpha/gbeta accumulate (caller
+ * zeroes), work = nblk*n + 2*nblk*ne floats.
+ * atsc3_wms_forward_work takes its workspace from the caller, nbp * (2n + ne)
+ * floats, nbp = nblk rounded up to a multiple of 4, and writes records (iters, nc,
+ * nbp), both 16-byte aligned; atsc3_wms_gradients reads those: the parameter
+ * gradients alone, gtot is only read, work = nbp*n + 2*nbp*ne floats. */
 int32_t atsc3_wms_forward_work(const int32_t *cptr, const int32_t *cidx,
                                const int32_t *vptr, const int32_t *vedge,
                                const int8_t *cbucket, int32_t n, int32_t nc,

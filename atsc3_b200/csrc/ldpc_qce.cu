@@ -2108,6 +2108,13 @@ int32_t atsc3_ldpc_qce_plan_create_one(int32_t n, int32_t kldpc, int32_t qa,
   return qce_plan_create_vb(n, kldpc, qa, qb, rowptr, addr, 0, 4, false, out);
 }
 
+int32_t atsc3_ldpc_qce_plan_create_one_f64(int32_t n, int32_t kldpc, int32_t qa,
+                                           int32_t qb, const int32_t *rowptr,
+                                           const int32_t *addr,
+                                           atsc3_ldpc_qce_plan **out) {
+  return qce_plan_create_vb(n, kldpc, qa, qb, rowptr, addr, 0, 8, false, out);
+}
+
 int32_t atsc3_ldpc_qce_plan_create_f64(int32_t n, int32_t kldpc, int32_t qa,
                                        int32_t qb, const int32_t *rowptr,
                                        const int32_t *addr, int32_t cluster,

@@ -152,14 +152,15 @@ class QcePlan(QcPlan):
         rowptr = np.ascontiguousarray(rowptr, np.int32)
         addr = np.ascontiguousarray(addr, np.int32)
         h = ctypes.c_void_p()
-        fn = ("atsc3_ldpc_qce_plan_create_f64" if dtype == "float64"
-              else "atsc3_ldpc_qce_plan_create2")
-        if cluster == 0 and not wide and dtype == "float32":
-            N.call("atsc3_ldpc_qce_plan_create_one", n, K, qa, qb,
+        f64 = dtype == "float64"
+        if cluster == 0 and not wide:
+            N.call("atsc3_ldpc_qce_plan_create_one_f64" if f64
+                   else "atsc3_ldpc_qce_plan_create_one", n, K, qa, qb,
                    rowptr.ctypes.data, addr.ctypes.data, ctypes.byref(h))
         else:
-            N.call(fn, n, K, qa, qb, rowptr.ctypes.data, addr.ctypes.data,
-                   int(cluster), ctypes.byref(h))
+            N.call("atsc3_ldpc_qce_plan_create_f64" if f64
+                   else "atsc3_ldpc_qce_plan_create2", n, K, qa, qb,
+                   rowptr.ctypes.data, addr.ctypes.data, int(cluster), ctypes.byref(h))
         self._h = h
         self.n, self.nc, self.dtype = n, n - K, dtype
         info = np.zeros(10, np.int64)

@@ -61,6 +61,8 @@ SIGNATURES = {
                                                c_vp, c_i32, c_vp]),
     "atsc3_ldpc_qce_plan_create_one": (c_i32, [c_i32, c_i32, c_i32, c_i32, c_vp,
                                                c_vp, c_vp]),
+    "atsc3_ldpc_qce_plan_create_one_f64": (c_i32, [c_i32, c_i32, c_i32, c_i32, c_vp,
+                                                   c_vp, c_vp]),
     "atsc3_ldpc_qce_plan_error": (c_i32, [c_vp, c_vp]),
     "atsc3_ldpc_qce_decode_f64": (c_i32, [c_vp, c_vp, c_i64, c_i32, c_i32, c_f64,
                                           c_i32, c_vp, c_i64, c_vp, c_i64, c_vp,

@@ -237,6 +237,11 @@ int32_t atsc3_ldpc_qce_plan_create_f64(int32_t n, int32_t kldpc, int32_t qa,
                                        int32_t qb, const int32_t *rowptr,
                                        const int32_t *addr, int32_t cluster,
                                        atsc3_ldpc_qce_plan **out);
+/* One cluster size for every batch, as atsc3_ldpc_qce_plan_create_one. */
+int32_t atsc3_ldpc_qce_plan_create_one_f64(int32_t n, int32_t kldpc, int32_t qa,
+                                           int32_t qb, const int32_t *rowptr,
+                                           const int32_t *addr,
+                                           atsc3_ldpc_qce_plan **out);
 int32_t atsc3_ldpc_qce_decode_f64(const atsc3_ldpc_qce_plan *plan, const double *llr,
                                   int64_t ld_llr, int32_t nblk, int32_t iters,
                                   double alpha, int32_t semantics, uint8_t *bits,
@@ -336,6 +341,9 @@ int32_t atsc3_ldpc_qce_spread_host(int32_t n, int32_t kldpc, int32_t qa, int32_t
                                    int32_t cluster, int32_t smax, int32_t *meta,
                                    int32_t *rdesc, int32_t *itab, int32_t *xtab);
 
+/* out: resident clusters, cluster size, shared memory per CTA and threads of the
+ * plan's own cluster size, which a decode of many codewords uses (a plan that
+ * holds larger sizes takes one of them for few). */
 int32_t atsc3_ldpc_qce_config(const atsc3_ldpc_qce_plan *plan, int32_t threads,
                               int32_t semantics, int32_t *out);
 

@@ -186,16 +186,17 @@ _PLANS = {}
 _PLANS_LOCK = threading.Lock()
 
 
-def plan_for(rate, n, dtype="float32", cluster=0, kind="auto"):
+def plan_for(rate, n, dtype="float32", cluster=0, kind="auto", wide=True):
     """Cached plan of an A/322 code.  kind "auto" picks the edge-buffer
     quasi-cyclic decoder (every code, float32 or float64), then in float32
     the record-layout one (Type B codes with one circulant per block),
     whichever first accepts the code; else the CSR decoder.  kind "qce" or
     "qc" asks for that decoder (raising if it rejects a code in its reach);
     codes outside its reach (float64 or Type A for "qc") get the CSR
-    decoder."""
+    decoder.  wide=False (edge-buffer plans): one cluster size for every
+    batch, for decodes that share the GPU (QcePlan)."""
     torch = _torch()
-    key = (rate, n, dtype, cluster, kind, torch.cuda.current_device())
+    key = (rate, n, dtype, cluster, kind, bool(wide), torch.cuda.current_device())
     with _PLANS_LOCK:
         p = _PLANS.get(key)
         if p is None:
@@ -204,7 +205,7 @@ def plan_for(rate, n, dtype="float32", cluster=0, kind="auto"):
             for k, cls, ok in (("qce", QcePlan, True), ("qc", QcPlan, f32 and type_b)):
                 if p is None and kind in ("auto", k) and ok:
                     try:
-                        p = (cls(rate, n, cluster=cluster, dtype=dtype) if k == "qce"
+                        p = (cls(rate, n, cluster=cluster, dtype=dtype, wide=wide) if k == "qce"
                              else cls(rate, n, cluster=cluster))
                     except N.FecError as e:
                         if kind == k or e.rc != -4:
@@ -290,7 +291,7 @@ def decode_flood(plan, llr, iters=50, alpha=0.75, semantics="kernel",
     return o
 
 
-def qce_plan_from_csr(tables, n, dtype="float32", cluster=0):
+def qce_plan_from_csr(tables, n, dtype="float32", cluster=0, wide=True):
     """The edge-buffer plan of the A/322 code whose CSR tables these are
     (atsc3_ldpc_qc_detect2: circulant structure, accumulator and identity
     parity, reference edge order), or None for any other matrix or a code
@@ -310,7 +311,7 @@ def qce_plan_from_csr(tables, n, dtype="float32", cluster=0):
     K, qa, qb = (int(x) for x in kq)
     nrows = K // 360 + (qa if qb else 0)
     try:
-        return QcePlan(dtype=dtype, cluster=cluster,
+        return QcePlan(dtype=dtype, cluster=cluster, wide=wide,
                        tables=(n, K, qa, qb, rowptr[:nrows + 1], addr[:rowptr[nrows]]))
     except N.FecError as e:
         if e.rc != -4:
@@ -325,12 +326,13 @@ class GpuMinSum:
     ``checks`` is the per-check column list (``m3_ldpc.parity_check``).
     ``decode(llr2d)`` takes (nblk, n) LLRs as numpy or a CUDA tensor and
     returns numpy ``(bits uint8, converged bool, iters int32, bad int32)``.
+    ``wide=False`` for a decoder that shares the GPU with others (QcePlan).
     """
 
     BIG = 1e9
 
     def __init__(self, checks, n, iters=50, alpha=0.75, device="cuda",
-                 dtype="float64", semantics="torch", cluster=0):
+                 dtype="float64", semantics="torch", cluster=0, wide=True):
         torch = _torch()
         if dtype not in ("float64", "float32", "bfloat16", "float16"):
             raise ValueError("dtype must be float64, float32, bfloat16 or float16")
@@ -356,7 +358,7 @@ class GpuMinSum:
             # edge-buffer decoder, any other matrix (and the narrow types)
             # the CSR decoder
             self.plan = None if narrow else qce_plan_from_csr(tabs, n, dtype=pdt,
-                                                              cluster=cluster)
+                                                              cluster=cluster, wide=wide)
             if self.plan is None:
                 self.plan = Plan(*tabs, n, dtype=pdt, cluster=cluster)
         self.nc = self.plan.nc

@@ -52,11 +52,13 @@ class FecPipeline:
     (this adds a host read of the flags).  ladder: None (the single `alpha`,
     as the configs pin it) or a tuple of alphas tried in turn on the blocks
     that did not converge (ldpc.ladder_decode; the reference's default
-    ladder is ldpc.ALPHA_LADDER)."""
+    ladder is ldpc.ALPHA_LADDER).  wide=False for a pipeline that shares the
+    GPU with others on other streams: few Blocks then take no more SMs a
+    Block than many do (ldpc.QcePlan)."""
 
     def __init__(self, n, mod, rate, iters=50, alpha=0.75, semantics="kernel",
                  cluster=0, threads=0, device="cuda", kind="auto",
-                 rescue=None, ladder=None):
+                 rescue=None, ladder=None, wide=True):
         torch = _torch()
         self.n, self.mod, self.rate = int(n), mod, rate
         self.nb = C.MOD_BITS[mod]
@@ -68,7 +70,7 @@ class FecPipeline:
         self.threads = threads
         self.device = torch.device(device)
         with torch.cuda.device(self.device):
-            self.plan = LDPC.plan_for(rate, n, "float32", cluster, kind=kind)
+            self.plan = LDPC.plan_for(rate, n, "float32", cluster, kind=kind, wide=wide)
             self.rescue = dict(rescue) if rescue else None
             self.ladder = tuple(ladder) if ladder else None
             self.sp_tab = (LDPC.sp_tables(C.csr(rate, n), n, self.device)

@@ -1,5 +1,6 @@
-"""QcePlan(wide=False): the plan keeps its one cluster size for every batch, in
-both value types, and decodes what a plan with larger sizes decodes."""
+"""wide=False: the plan keeps its one cluster size for every batch, in both value
+types and through every entry point that builds one, and decodes what a plan
+with larger sizes decodes."""
 import numpy as np
 import pytest
 
@@ -34,3 +35,22 @@ def test_one_size_decodes_alike(dtype):
         a, b = (ldpc.decode_flood(p, x[:nblk], iters=20) for p in (one, wide))
         for k in ("bits", "conv", "its", "bad"):
             assert np.array_equal(a[k].cpu().numpy(), b[k].cpu().numpy()), (nblk, k)
+
+
+@pytest.mark.gpu
+def test_wide_reaches_the_plan(monkeypatch):
+    from atsc3_b200 import codes as C
+    from atsc3_b200.pipeline import FecPipeline
+    made, real = [], ldpc.QcePlan
+    monkeypatch.setattr(ldpc, "QcePlan",
+                        lambda *a, **kw: (made.append(kw["wide"]), real(*a, **kw))[1])
+    monkeypatch.setattr(ldpc, "_PLANS", {})
+    tabs = C.csr("6/15", 16200)
+    checks = np.split(tabs[1], tabs[0][1:-1])
+    for make in (lambda **kw: ldpc.plan_for("6/15", 16200, **kw),
+                 lambda **kw: ldpc.qce_plan_from_csr(tabs, 16200, **kw),
+                 lambda **kw: FecPipeline(16200, "QPSK", "9/15", **kw).plan,
+                 lambda **kw: ldpc.GpuMinSum(checks, 16200, **kw).plan):
+        made.clear()
+        plans = [make(), make(wide=False)]
+        assert made == [True, False] and plans[0] is not plans[1]

@@ -1296,7 +1296,8 @@ __device__ __forceinline__ int qce_claim(int32_t *its, int nblk, int guess, int 
     if (__shfl_sync(0xffffffffu, old, 0) == -1) return guess;
   }
   int p = *base, got = -1;
-  while (got < 0 && p < nblk) {
+  // a claim that fails means one made by another cluster, so fewer than nblk fail
+  for (int fails = 0; got < 0 && p < nblk && fails < nblk;) {
     int v[8];                       // 256 codewords a round trip
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -1318,9 +1319,8 @@ __device__ __forceinline__ int qce_claim(int32_t *its, int nblk, int guess, int 
     p += 32 * w;
     const int k = p + (int)__fns(open, 0, 1 + (int)(cluster_id_x() % (uint32_t)__popc(open)));
     if (lane == 0) old = atomicCAS(its + k, -1, -2);
-    // where it failed another cluster has taken it since the look: at most one
-    // more look per codeword
     if (__shfl_sync(0xffffffffu, old, 0) == -1) got = k;
+    else ++fails;
   }
   __syncwarp();
   if (lane == 0) *base = p;

@@ -41,3 +41,18 @@ def test_outputs_held_anything_two_streams(rate, n, nblk):
             for k in KEYS:
                 assert torch.equal(o[k], w[k]), (poison, k)
 
+
+def test_status_outputs_in_pinned_host_memory():
+    import torch
+    from atsc3_b200.ldpc import QcePlan, decode_flood
+    plan = QcePlan("9/15", 16200)
+    x = _llr(torch, 200, 16200, 4)
+    want = decode_flood(plan, x, iters=30)
+    out = {k: torch.full_like(want[k], 77, device="cpu").pin_memory() for k in ("conv", "its", "bad")}
+    for _ in range(3):
+        got = decode_flood(plan, x, iters=30, out=dict(out))
+        torch.cuda.synchronize()
+        assert torch.equal(got["bits"], want["bits"])
+        for k in out:
+            assert torch.equal(out[k], want[k].cpu()), k
+            out[k].fill_(-1 if k != "conv" else 1)

@@ -390,10 +390,13 @@ int32_t atsc3_cpe_correct(const double *pool, int64_t ncells,
   a.nparts = nparts;
   cpe_power_kernel<<<nparts, CPE_T, 0, st>>>(a);
   const int smem = 3 * 4 * (cpe_padded(m0) + cpe_padded(m1));
-  if (smem > 48 * 1024)
+  // 4096 points are 48 KB by themselves, and the kernel's static shared memory
+  // counts towards the 48 KB that a launch gets without asking.  Every caller asks
+  // for the largest alphabets' size, so none lowers another thread's limit.
+  if (smem > 40 * 1024)
     ATSC3_CUDA(cudaFuncSetAttribute((const void *)cpe_symbol_kernel,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    smem));
+                                    3 * 4 * 2 * 4096));
   // CTAs per symbol: what it takes to have four CTAs on every SM (their
   // registers' limit), as long as each keeps a cell for every thread
   // (61 symbols of 19949 cells: 8 CTAs each 151 us, 7 164, 6 at three an SM 148;

@@ -32,9 +32,15 @@ constexpr int DEMAP_T = 256;    // threads per CTA, a cell each
 // CTAs per SM the compiler has to leave room for: the fully unrolled 64- and
 // 256-point kernels run best with just the registers of four (75 x 64800-bit
 // Blocks: 64 points 31.2 us without the bound, 23.0 with it; 256 points 37.4
-// and 31.6; 16 points and the grids lose by it)
+// and 31.6; the grids lose by it).  16 points are bound by memory latency and the
+// scattered stores, so by the warps in flight (codeword order, one sigma2 / one per
+// cell: 16.9 / 18.4 us without the bound, which takes 62 registers, 15.5 / 16.8 with
+// five CTAs, 14.5 / 15.6 with six, 13.8 / 14.7 with eight, which do not spill; 13.0 /
+// 14.0 with one 32-bit division a cell instead of a 64-bit one and a 32-bit one).
 template <int NB, typename T>
-constexpr int demap_ctas() { return sizeof(T) == 4 && (NB == 6 || NB == 8) ? 4 : 1; }
+constexpr int demap_ctas() {
+  return sizeof(T) != 4 ? 1 : NB == 4 ? 8 : NB == 6 || NB == 8 ? 4 : 1;
+}
 
 // Writes one cell's LLRs: through lam_of_q (nullable) or in transmission
 // order, the table and the contiguous LLRs in the widest aligned pieces.
@@ -104,11 +110,19 @@ __global__ void __launch_bounds__(DEMAP_T, (demap_ctas<NB, T>())) demap_kernel(
   const int64_t total = (int64_t)nblk * ncell;
   for (int64_t g0 = (int64_t)blockIdx.x * DEMAP_T; g0 < total;
        g0 += (int64_t)gridDim.x * DEMAP_T) {
-    // the CTA's first cell, then a 32-bit step from it
-    const int64_t b0 = g0 / ncell;
-    const uint32_t x = (uint32_t)(g0 - b0 * ncell) + threadIdx.x;
+    // row and cell: one 32-bit division where the batch allows it, else the CTA's
+    // first cell and a 32-bit step from it
+    int64_t b;
+    uint32_t x = threadIdx.x;
+    if (total <= 0xFFFFFFFFll - DEMAP_T) {
+      x += (uint32_t)g0;
+      b = 0;
+    } else {
+      b = g0 / ncell;
+      x += (uint32_t)(g0 - b * ncell);
+    }
     const uint32_t step = x / (uint32_t)ncell;
-    const int64_t b = b0 + step;
+    b += step;
     const int s = (int)(x - step * (uint32_t)ncell);
     if (b >= nblk) break;
     const typename Cell2<T>::type z = cells[(size_t)b * ld_cells + s];

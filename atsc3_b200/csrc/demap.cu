@@ -424,55 +424,6 @@ int32_t demap_f64_launch(const double *cells, int64_t ld_cells, int nblk,
   return 0;
 }
 
-// CTAs a row of the estimating pass: what fills the chip, at most the row's
-// cells and the 4096 sums the workspace holds beyond one per row.
-template <int NB, typename T>
-static int32_t demap_estimate_nb(const T *cells, int64_t ld_cells, int nblk, int ncell,
-                                 const T *pts, const int32_t *lam_of_q, T *out,
-                                 int64_t ld_out, double *work, cudaStream_t st) {
-  using T2 = typename Cell2<T>::type;
-  auto *fn = demap_sum_kernel<NB, T>;
-  const int smem = demap_smem_bytes(NB, sizeof(T));
-  if (smem > 48 * 1024)
-    ATSC3_CUDA(cudaFuncSetAttribute((const void *)fn,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  const int full = std::max(1, std::min(4096, num_sms() * demap_waves(NB)) / nblk);
-  const int chunks = std::min((ncell + DEMAP_T - 1) / DEMAP_T, full);
-  fn<<<nblk * chunks, DEMAP_T, smem, st>>>((const T2 *)cells, ld_cells, ncell, chunks, pts,
-                                           lam_of_q, out, ld_out, work);
-  ATSC3_CUDA(cudaGetLastError());
-  const int width = ncell * NB;
-  const int wide = std::max(1, std::min((width + 4 * DEMAP_T - 1) / (4 * DEMAP_T),
-                                        num_sms() * 8 / nblk));
-  demap_scale_kernel<T><<<nblk * wide, DEMAP_T, 0, st>>>(work, chunks, ncell, wide, width, out,
-                                                        ld_out);
-  ATSC3_CUDA(cudaGetLastError());
-  return 0;
-}
-
-template <typename T>
-static int32_t demap_estimate_launch(const T *cells, int64_t ld_cells, int nblk, int ncell,
-                                     const T *pts, int nbits, const int32_t *lam_of_q, T *out,
-                                     int64_t ld_out, void *work, cudaStream_t st) {
-  ATSC3_ARG(nbits >= 2 && nbits <= 12 && nbits % 2 == 0, "nbits must be 2, 4, 6, 8, 10 or 12");
-  ATSC3_ARG(nblk >= 0 && ncell > 0, "bad size");
-  if (nblk == 0) return 0;
-  ATSC3_ARG(cells && pts && out && work, "null pointer");
-  ATSC3_ARG(ld_cells >= ncell, "ld_cells < ncell");
-  ATSC3_ARG(ld_out >= (int64_t)ncell * nbits, "ld_out < ncell*nbits");
-  ATSC3_ARG((int64_t)ncell * nbits <= INT32_MAX, "a row of more than 2^31 - 1 LLRs");
-  ATSC3_ARG(((uintptr_t)cells & (2 * sizeof(T) - 1)) == 0, "cells must be aligned to a cell");
-  double *w = (double *)work;
-  switch (nbits) {
-    case 2: return demap_estimate_nb<2, T>(cells, ld_cells, nblk, ncell, pts, lam_of_q, out, ld_out, w, st);
-    case 4: return demap_estimate_nb<4, T>(cells, ld_cells, nblk, ncell, pts, lam_of_q, out, ld_out, w, st);
-    case 6: return demap_estimate_nb<6, T>(cells, ld_cells, nblk, ncell, pts, lam_of_q, out, ld_out, w, st);
-    case 8: return demap_estimate_nb<8, T>(cells, ld_cells, nblk, ncell, pts, lam_of_q, out, ld_out, w, st);
-    case 10: return demap_estimate_nb<10, T>(cells, ld_cells, nblk, ncell, pts, lam_of_q, out, ld_out, w, st);
-    default: return demap_estimate_nb<12, T>(cells, ld_cells, nblk, ncell, pts, lam_of_q, out, ld_out, w, st);
-  }
-}
-
 int32_t row_sigma_f64_launch(const double *cells, int64_t ld_cells, int nblk,
                              int ncell, const double *pts, int nbits,
                              double *sigma2, cudaStream_t st) {
@@ -512,6 +463,85 @@ int32_t row_sigma_launch(const float *cells, int64_t ld_cells, int nblk,
                               sigma2);
   ATSC3_CUDA(cudaGetLastError());
   return 0;
+}
+
+// CTAs a row of the estimating pass: what fills the chip, at most the row's
+// cells and the 4096 sums the workspace holds beyond one per row.
+template <int NB, typename T>
+static int32_t demap_estimate_nb(const T *cells, int64_t ld_cells, int nblk, int ncell,
+                                 const T *pts, const int32_t *lam_of_q, T *out,
+                                 int64_t ld_out, double *work, cudaStream_t st) {
+  using T2 = typename Cell2<T>::type;
+  auto *fn = demap_sum_kernel<NB, T>;
+  const int smem = demap_smem_bytes(NB, sizeof(T));
+  if (smem > 48 * 1024)
+    ATSC3_CUDA(cudaFuncSetAttribute((const void *)fn,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  const int full = std::max(1, std::min(4096, num_sms() * demap_waves(NB)) / nblk);
+  const int chunks = std::min((ncell + DEMAP_T - 1) / DEMAP_T, full);
+  fn<<<nblk * chunks, DEMAP_T, smem, st>>>((const T2 *)cells, ld_cells, ncell, chunks, pts,
+                                           lam_of_q, out, ld_out, work);
+  ATSC3_CUDA(cudaGetLastError());
+  const int width = ncell * NB;
+  const int wide = std::max(1, std::min((width + 4 * DEMAP_T - 1) / (4 * DEMAP_T),
+                                        num_sms() * 8 / nblk));
+  demap_scale_kernel<T><<<nblk * wide, DEMAP_T, 0, st>>>(work, chunks, ncell, wide, width, out,
+                                                        ld_out);
+  ATSC3_CUDA(cudaGetLastError());
+  return 0;
+}
+
+// Many short rows: one pass over the rows for the estimates and one over all cells
+// for the LLRs.  A row's own CTA in both passes leaves most threads idle below 256
+// cells, and QPSK's minima cost less than reading its LLRs back (us, one pass that
+// is divided after / two passes, float32: 6666 rows of 30 cells, QPSK 23.0 / 10.9,
+// 64 points 31.6 / 18.8; 1562 of 128, 9.1 / 6.5 and 13.1 / 11.8; 778 of 257, 256
+// points 21.0 / 21.6; QPSK 1481 of 1350 cells 19.5 / 16.6).
+static bool demap_short_rows(int nblk, int ncell, int nbits) {
+  return nblk >= num_sms() && (ncell <= 256 || (nbits == 2 && ncell <= 4096));
+}
+
+static int32_t demap_short(const float *cells, int64_t ld_cells, int nblk, int ncell,
+                           const float *pts, int nbits, const int32_t *lam_of_q, float *out,
+                           int64_t ld_out, void *work, cudaStream_t st) {
+  float *s2 = (float *)work;
+  const int32_t rc = row_sigma_launch(cells, ld_cells, nblk, ncell, pts, nbits, s2, st);
+  return rc ? rc : demap_launch(cells, ld_cells, nblk, ncell, pts, nbits, 2, s2, 0, 1.f, lam_of_q,
+                                out, ld_out, st);
+}
+
+static int32_t demap_short(const double *cells, int64_t ld_cells, int nblk, int ncell,
+                           const double *pts, int nbits, const int32_t *lam_of_q, double *out,
+                           int64_t ld_out, void *work, cudaStream_t st) {
+  double *s2 = (double *)work;
+  const int32_t rc = row_sigma_f64_launch(cells, ld_cells, nblk, ncell, pts, nbits, s2, st);
+  return rc ? rc : demap_f64_launch(cells, ld_cells, nblk, ncell, pts, nbits, 2, s2, 0, 1.0,
+                                    lam_of_q, out, ld_out, st);
+}
+
+template <typename T>
+static int32_t demap_estimate_launch(const T *cells, int64_t ld_cells, int nblk, int ncell,
+                                     const T *pts, int nbits, const int32_t *lam_of_q, T *out,
+                                     int64_t ld_out, void *work, cudaStream_t st) {
+  ATSC3_ARG(nbits >= 2 && nbits <= 12 && nbits % 2 == 0, "nbits must be 2, 4, 6, 8, 10 or 12");
+  ATSC3_ARG(nblk >= 0 && ncell > 0, "bad size");
+  if (nblk == 0) return 0;
+  ATSC3_ARG(cells && pts && out && work, "null pointer");
+  ATSC3_ARG(ld_cells >= ncell, "ld_cells < ncell");
+  ATSC3_ARG(ld_out >= (int64_t)ncell * nbits, "ld_out < ncell*nbits");
+  ATSC3_ARG((int64_t)ncell * nbits <= INT32_MAX, "a row of more than 2^31 - 1 LLRs");
+  ATSC3_ARG(((uintptr_t)cells & (2 * sizeof(T) - 1)) == 0, "cells must be aligned to a cell");
+  if (demap_short_rows(nblk, ncell, nbits))
+    return demap_short(cells, ld_cells, nblk, ncell, pts, nbits, lam_of_q, out, ld_out, work, st);
+  double *w = (double *)work;
+  switch (nbits) {
+    case 2: return demap_estimate_nb<2, T>(cells, ld_cells, nblk, ncell, pts, lam_of_q, out, ld_out, w, st);
+    case 4: return demap_estimate_nb<4, T>(cells, ld_cells, nblk, ncell, pts, lam_of_q, out, ld_out, w, st);
+    case 6: return demap_estimate_nb<6, T>(cells, ld_cells, nblk, ncell, pts, lam_of_q, out, ld_out, w, st);
+    case 8: return demap_estimate_nb<8, T>(cells, ld_cells, nblk, ncell, pts, lam_of_q, out, ld_out, w, st);
+    case 10: return demap_estimate_nb<10, T>(cells, ld_cells, nblk, ncell, pts, lam_of_q, out, ld_out, w, st);
+    default: return demap_estimate_nb<12, T>(cells, ld_cells, nblk, ncell, pts, lam_of_q, out, ld_out, w, st);
+  }
 }
 
 // ---- uneven batches: every block its own constellation ---------------------

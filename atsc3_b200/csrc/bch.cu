@@ -138,10 +138,15 @@ __global__ void __launch_bounds__(BCH_T) bch_bits_kernel(
   reduce_store(acc, syn + (size_t)b * 6, nullptr);
 }
 
-// CTAs per codeword: few words a warp while that leaves a few CTAs per SM.
+// CTAs per codeword: as many as leave the whole batch resident at once, which is
+// three CTAs an SM by their registers, and two in clusters of eight (us with 1 / 2 /
+// 4 / 8 CTAs a codeword: 37 of 64800 6/15 16.9 / 10.4 / 7.1 / 5.9, 74 17.4 / 10.8 /
+// 8.3 / 10.1, 148 18.1 / 11.3 / 15.1 / 17.4, 300 20.4 / 23.2 / 22.1 / 30.2; 148 of
+// 16200 2/15 5.2 / 4.5 / 7.2 / 11.2).
 static int bch_cluster(int64_t nblk, int kldpc) {
   int cl = BCH_CL;
-  while (cl > 1 && (nblk * cl > 8 * 148 || kldpc / 32 < cl * (BCH_T / 32))) cl /= 2;
+  const auto room = [](int c) { return c == 8 ? 2 * 148 : c == 4 ? 400 : 3 * 148; };
+  while (cl > 1 && (nblk * cl > room(cl) || kldpc / 32 < cl * (BCH_T / 32))) cl /= 2;
   return cl;
 }
 

@@ -14,7 +14,7 @@
 // distributed shared memory.  The table sits in L2; with one CTA a codeword and a
 // word a thread, its latency and the 32 lines each load touched were the bound
 // (one 16200 11/15 codeword 13.3 us, 7 of 64800 10/15 37.8, 75 of 6/15 26.6; now
-// 3.6, 5.8 and 9.8).
+// 3.6, 5.8 and 8.3).
 // The descrambled payload (lab/m9_fast.py:942-949: hard bits XOR the
 // scrambling sequence, packed MSB-first) is written by the same cluster.
 

@@ -181,8 +181,8 @@ template <> struct DemapArith<double> {
 // (measured: fma.rn.f32x2 with three register operands 3.0 cycles, with one
 // from constant memory 2.0; a three-operand minimum 2.0).  75 Blocks of 64800
 // bits with per-cell sigma2, before (one metric and five minima a label) and
-// now: 64 points 31.0 -> 22.6 us, 256 points 70.2 -> 31.4, 1024 points 187 ->
-// 35.4, 4096 points 625 -> 39.5.
+// now, launches back to back: 16 points 15.9 -> 14.0 us, 64 points 28.2 -> 19.8,
+// 256 points 67.4 -> 29.6, 1024 points 184 -> 33.6, 4096 points 621 -> 37.7.
 enum DemapForm { FORM_GENERAL = 0, FORM_STRUCT = 1 };
 
 // the minima of the four low label bits, from those of 16 columns

@@ -1281,13 +1281,17 @@ __device__ __forceinline__ int qce_check_heavy(const uint2 *he, int deg, int wra
 // another cluster; cancelling clusters not yet launched (clusterlaunchcontrol)
 // gains the same but needs a wait for the answer, and a codeword whose answer does
 // not come within a bounded wait is decoded by nobody.  Against fixed shares, ms:
-// 66 codewords of 64800 8/15, a few of them at 50 iterations, 1.168 -> 0.796; three
+// 45 codewords of 64800 8/15, a few of them at 50 iterations, in a decode chain 1.303 ->
+// 1.129, 66 of them decoded 1.168 -> 0.796; three
 // codewords a cluster that all end alike, 64800 4/15 1.056 -> 1.058, 13/15 0.481 ->
 // 0.488 (0.494 with one window of 32 words a round trip in the search).
 // The codeword that a fixed share would hold next is tried first, one round trip
 // to the L2 that the outputs' stores cover; where it is taken, the first word with
 // an open codeword is searched, clusters that search at once trying different
-// ones of it.  Every lane of one warp calls it; `base`: everything below is taken.
+// ones of it.  So a batch of even codewords runs as fixed shares do.  (The search
+// alone, in ascending order: 12 seeds of those 45-codeword chains 1.003 ms on
+// average, 1.010 here; 222 even ones of 16200 3/15 0.724 ms, 0.705 here.)  Every lane
+// of one warp calls it; `base`: everything below is taken.
 __device__ __forceinline__ int qce_claim(int32_t *its, int nblk, int guess, int *base) {
   const int lane = threadIdx.x & 31;
   int old = 0;

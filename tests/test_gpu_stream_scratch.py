@@ -37,25 +37,42 @@ def _sp(torch, _):
 @pytest.mark.parametrize("make,dtype", [(_demap, "complex64"), (_demap, "complex128"),
                                         (_cpe, None), (_sp, None)])
 def test_scratch_stays_until_the_stream_has_run(make, dtype, monkeypatch):
+    import ctypes
+    import gc
+
     import torch
     from atsc3_b200 import native as N
     call = make(torch, getattr(torch, dtype) if dtype else None)
     side = torch.cuda.Stream()
+    sizes, empty = [], torch.empty
+
+    def noted(*a, **kw):
+        t = empty(*a, **kw)
+        sizes.append(t.nbytes)
+        return t
+
+    monkeypatch.setattr(torch, "empty", noted)
     call(0)                                     # the default stream; tables and modules loaded
+    monkeypatch.setattr(torch, "empty", empty)
+    # the memory that is asked for below is there before the stream is held up, so
+    # that nothing waits for the device meanwhile
+    gc.collect()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    held = [[torch.empty(n, dtype=torch.uint8, device="cuda") for _ in range(8)] for n in sizes]
+    torch.cuda._sleep(1000)
     torch.cuda.synchronize()
     scratch, real = [], N.call
     monkeypatch.setattr(N, "call", lambda name, *a: (scratch.append(a[-2]), real(name, *a))[1]
                         if name.startswith(("atsc3_demap_est", "atsc3_cpe_corr", "atsc3_ldpc_sp_dec"))
                         else real(name, *a))
     with torch.cuda.stream(side):
-        torch.cuda._sleep(400_000_000)          # about a fifth of a second
-    import ctypes
+        torch.cuda._sleep(2_000_000_000)        # about a second
     for handle in (side.cuda_stream, ctypes.c_void_p(side.cuda_stream)):
         call(handle)
-    fresh = [torch.empty(size, dtype=torch.uint8, device="cuda")
-             for size in (4096 * 8, 1 << 20, 1 << 21, 1 << 16) for _ in range(12)]
-    pending = not side.query()
-    assert pending and len(scratch) == 2
+    del held
+    fresh = [torch.empty(n, dtype=torch.uint8, device="cuda") for n in sizes for _ in range(40)]
+    assert not side.query() and len(scratch) == 2
     for t in fresh:
         lo, hi = t.data_ptr(), t.data_ptr() + t.numel()
         assert not any(lo <= s < hi for s in scratch)
